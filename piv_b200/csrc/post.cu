@@ -8,8 +8,11 @@
 // statistics use a fixed-order tree and agree to f32 rounding.
 #include <algorithm>
 #include <cmath>
+#include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -52,77 +55,139 @@ __device__ __forceinline__ bool deriv(const float* d, const float* dxf, const ui
     return true;
 }
 
-__global__ void flow_kernel(int ny, int nx, float k, float h, const float* __restrict__ dx, const float* __restrict__ dy,
-                            const uint8_t* __restrict__ fl, float* vort, FlowPartial* part) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double ws = 0.0, wa = 0.0, e = 0.0;
-    long long nw = 0, n = 0;
-    if (i < ny * nx) {
-        const int iy = i / nx, ix = i % nx;
+// One launch per field: every block sums its cells in a fixed order, and the block that finishes
+// last adds the block sums in block order and writes the result to mapped host memory, so a call is
+// one kernel and one stream wait. It is bound by that launch-and-wait latency, not by its 9 bytes
+// per cell. The block sums live in a fixed set of device slots: allocating them per call made the
+// stream-ordered pool map and unmap memory at every wait, and one thread added the block sums
+// (64 fields of 118 x 66 smoothed and summed: 30-60 -> 1.7 ms, B200).
+constexpr int kFlowThreads = 256;
+constexpr int kFlowBlocks = 296;  // two per SM; larger fields loop
+constexpr int kFlowSlots = 16;    // calls in flight per device; further callers wait for a slot
+constexpr int kFlowMaxDevices = 16;
+
+struct FlowSlot {
+    FlowPartial part[kFlowBlocks];
+    unsigned int done;  // blocks finished; the last one sets it back to 0
+};
+__device__ FlowSlot g_flow[kFlowSlots];
+
+// Sum over the block in a fixed order; the result is valid in thread 0.
+__device__ __forceinline__ FlowPartial flow_block_sum(FlowPartial p) {
+    __shared__ FlowPartial sh[kFlowThreads / 32];
+    auto add_from = [&](int o) {
+        p.ws += __shfl_down_sync(0xffffffffu, p.ws, o);
+        p.wa += __shfl_down_sync(0xffffffffu, p.wa, o);
+        p.e += __shfl_down_sync(0xffffffffu, p.e, o);
+        p.nw += __shfl_down_sync(0xffffffffu, p.nw, o);
+        p.n += __shfl_down_sync(0xffffffffu, p.n, o);
+    };
+    for (int o = 16; o > 0; o >>= 1) add_from(o);
+    if (threadIdx.x % 32 == 0) sh[threadIdx.x / 32] = p;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        p = threadIdx.x < kFlowThreads / 32 ? sh[threadIdx.x] : FlowPartial{0.0, 0.0, 0.0, 0, 0};
+        for (int o = kFlowThreads / 64; o > 0; o >>= 1) add_from(o);
+    }
+    __syncthreads();  // sh may be written again
+    return p;
+}
+
+__global__ void __launch_bounds__(kFlowThreads) flow_kernel(int ny, int nx, float k, float h,
+                                                            const float* __restrict__ dx, const float* __restrict__ dy,
+                                                            const uint8_t* __restrict__ fl, float* vort, int slot,
+                                                            FlowPartial* out) {
+    FlowPartial t{0.0, 0.0, 0.0, 0, 0};
+    const long long cells = (long long)ny * nx;
+    for (long long c = (long long)blockIdx.x * kFlowThreads + threadIdx.x; c < cells; c += (long long)gridDim.x * kFlowThreads) {
+        const int i = (int)c, iy = i / nx, ix = i % nx;
         float a, b;
         const bool ha = deriv(dx, dx, fl, iy, ny, i, nx, k, h, &a);  // du/dy
         const bool hb = deriv(dy, dx, fl, ix, nx, i, 1, k, h, &b);   // dv/dx
         const float w = (ha && hb) ? __fsub_rn(a, b) : NAN;
         if (vort) vort[i] = w;
         if (isfinite(w)) {
-            ws = (double)w;
-            wa = (double)fabsf(w);
-            nw = 1;
+            t.ws += (double)w;
+            t.wa += (double)fabsf(w);
+            ++t.nw;
         }
         const float u = __fmul_rn(dx[i], k), v = __fmul_rn(dy[i], k);
         if (usable_cell(dx[i], fl[i]) && isfinite(u) && isfinite(v)) {
-            e = 0.5 * __dadd_rn(__dmul_rn((double)u, (double)u), __dmul_rn((double)v, (double)v));
-            n = 1;
+            t.e += 0.5 * __dadd_rn(__dmul_rn((double)u, (double)u), __dmul_rn((double)v, (double)v));
+            ++t.n;
         }
     }
-    // fixed-order block reduction
-    __shared__ FlowPartial sh[256];
-    sh[threadIdx.x] = FlowPartial{ws, wa, e, nw, n};
+    t = flow_block_sum(t);
+    FlowSlot& s = g_flow[slot];
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        s.part[blockIdx.x] = t;
+        __threadfence();
+        last = atomicAdd(&s.done, 1u) == gridDim.x - 1;
+    }
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) {
-            FlowPartial& p = sh[threadIdx.x];
-            const FlowPartial& q = sh[threadIdx.x + s];
-            p.ws += q.ws;
-            p.wa += q.wa;
-            p.e += q.e;
-            p.nw += q.nw;
-            p.n += q.n;
-        }
-        __syncthreads();
+    if (!last) return;
+    __threadfence();
+    t = FlowPartial{0.0, 0.0, 0.0, 0, 0};
+    for (int j = threadIdx.x; j < (int)gridDim.x; j += kFlowThreads) {
+        const volatile FlowPartial& q = s.part[j];
+        t.ws += q.ws;
+        t.wa += q.wa;
+        t.e += q.e;
+        t.nw += q.nw;
+        t.n += q.n;
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+    t = flow_block_sum(t);
+    if (threadIdx.x == 0) {
+        s.done = 0;
+        *out = t;
+    }
 }
 
-__global__ void flow_final_kernel(const FlowPartial* part, int nparts, FlowPartial* out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    FlowPartial t{0.0, 0.0, 0.0, 0, 0};
-    for (int j = 0; j < nparts; ++j) {
-        t.ws += part[j].ws;
-        t.wa += part[j].wa;
-        t.e += part[j].e;
-        t.nw += part[j].nw;
-        t.n += part[j].n;
-    }
-    *out = t;
-}
+// Slots of flow_kernel per device: a call holds one from its launch to the end of its wait. The
+// mapped host block (one result per slot) is made once per process and shared by all devices.
+static std::mutex g_flow_mu;
+static std::condition_variable g_flow_cv;
+static std::map<int, unsigned int> g_flow_used;  // device -> slots in use
+static FlowPartial* g_flow_host = nullptr;       // kFlowSlots results
 
 cudaError_t flow_stats_device(int ny, int nx, float step, double dt_s, const float* dx, const float* dy,
                               const uint8_t* flags, float* vort, FlowStatsHost* stats, cudaStream_t s) {
     const int cells = ny * nx;
-    const int blocks = (cells + 255) / 256;
-    void* buf = nullptr;
-    cudaError_t e = cudaMallocAsync(&buf, sizeof(FlowPartial) * (size_t)(blocks + 1), s);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    FlowPartial* part = static_cast<FlowPartial*>(buf);
-    const float k = (float)(1.0 / dt_s);
-    flow_kernel<<<blocks, 256, 0, s>>>(ny, nx, k, step, dx, dy, flags, vort, part);
-    flow_final_kernel<<<1, 32, 0, s>>>(part, blocks, part + blocks);
-    FlowPartial t{};
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&t, part + blocks, sizeof(t), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(buf, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    int slot = 0;
+    {
+        std::unique_lock<std::mutex> lk(g_flow_mu);
+        if (!g_flow_host) {
+            void* m = nullptr;
+            e = cudaHostAlloc(&m, sizeof(FlowPartial) * kFlowSlots * kFlowMaxDevices, cudaHostAllocPortable | cudaHostAllocMapped);
+            if (e != cudaSuccess) return e;
+            g_flow_host = static_cast<FlowPartial*>(m);
+        }
+        if (dev >= kFlowMaxDevices) return cudaErrorInvalidDevice;
+        unsigned int& used = g_flow_used[dev];
+        g_flow_cv.wait(lk, [&] { return used != (1u << kFlowSlots) - 1; });
+        while (used >> slot & 1u) ++slot;
+        used |= 1u << slot;
+    }
+    FlowPartial* host = g_flow_host + dev * kFlowSlots + slot;
+    FlowPartial* out = nullptr;
+    e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&out), host, 0);
+    if (e == cudaSuccess) {
+        const int blocks = std::min((cells + kFlowThreads - 1) / kFlowThreads, kFlowBlocks);
+        flow_kernel<<<blocks, kFlowThreads, 0, s>>>(ny, nx, (float)(1.0 / dt_s), step, dx, dy, flags, vort, slot, out);
+        e = cudaGetLastError();
+        const cudaError_t w = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = w;
+    }
+    const FlowPartial t = *host;
+    {
+        std::lock_guard<std::mutex> lk(g_flow_mu);
+        g_flow_used[dev] &= ~(1u << slot);
+    }
+    g_flow_cv.notify_one();
     if (e != cudaSuccess) return e;
     auto mean = [](double v, long long c) { return c > 0 ? (float)(v / (double)c) : NAN; };
     stats->vorticity_mean = mean(t.ws, t.nw);
