@@ -159,6 +159,7 @@ struct PivFrame {
     int* scales = nullptr;
     unsigned int* words = nullptr;  // maxbits[2] + histogram scratch
     bool stats_valid = false;
+    bool strips = true;  // how the tables are stored (StatsView)
     bool nonneg = false;
     void* d_raw = nullptr;
     size_t d_raw_bytes = 0;
@@ -282,7 +283,7 @@ int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
     return PIV_OK;
 }
 
-StatsView stats_of(const PivFrame* f) { return StatsView{f->sum, f->sumsq, f->scales, (int)f->H, (int)f->W}; }
+StatsView stats_of(const PivFrame* f) { return StatsView{f->sum, f->sumsq, f->scales, (int)f->H, (int)f->W, f->strips}; }
 
 bool needs_stats(const PivAnalyzer* an, const PivFrame* f) { return !an->mask_trivial() || !f->nonneg; }
 
@@ -460,7 +461,8 @@ int run_passes(PivAnalyzer* an, const PivFrame* const* a, const PivFrame* const*
     for (int k = 0; k < K; ++k)
         for (const PivFrame* f : {a[k], b[k]})
             for (uintptr_t v : {(uintptr_t)f, (uintptr_t)f->image, (uintptr_t)f->sum, (uintptr_t)f->sumsq,
-                                (uintptr_t)f->scales, (uintptr_t)needs_stats(an, f), (uintptr_t)f->stats_valid})
+                                (uintptr_t)f->scales, (uintptr_t)needs_stats(an, f), (uintptr_t)f->stats_valid,
+                                (uintptr_t)f->strips})
                 key.push_back(v);
     if (an->gexec && key == an->gkey) {
         CUDA_TRY(cudaGraphLaunch(an->gexec, an->cur));
@@ -574,6 +576,7 @@ int prepare_common(PivAnalyzer* an, PivFrame* f, const void* raw_dev, int32_t dt
     CUDA_TRY(launch_prepare(pp, an->cur, &nl));
     an->launches += nl;
     f->stats_valid = stats;
+    f->strips = true;
     return PIV_OK;
 }
 
@@ -864,6 +867,7 @@ int32_t piv_frame_set_prepared(PivAnalyzer* an, PivFrame* f, const float* image,
     CUDA_TRY(launch_stats(bsrc, (int)f->H, (int)f->W, f->sum, f->sumsq, f->scales, f->words, an->cur, &nl));
     an->launches += nl;
     f->stats_valid = true;
+    f->strips = true;
     CUDA_TRY(cudaStreamSynchronize(an->cur));
     return PIV_OK;
 }
@@ -878,6 +882,7 @@ int32_t piv_frame_set_prepared_tables(PivAnalyzer* an, PivFrame* f, const float*
     const size_t cells = (size_t)(f->H + 1) * (size_t)(f->W + 1);
     CUDA_TRY(cudaMemcpyAsync(f->image, image, sizeof(float) * n, cudaMemcpyHostToDevice, an->cur));
     f->nonneg = false;  // unknown: statistics are always used
+    f->strips = false;
     st = alloc_stats(f);
     if (st) return st;
     // the f64 tables land in the int64 tables' storage (8 bytes per entry) and are converted there

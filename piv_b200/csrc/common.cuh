@@ -144,6 +144,14 @@ __device__ __forceinline__ long long fix_q2(float v, const FixScale& fs) {
     return __float2ll_rn(scalbnf(sq.hi, fs.s2)) + __float2ll_rn(scalbnf(sq.lo, fs.s2));
 }
 
+// Entry (y, x) of an integral table stored in strips: rows that are multiples of kStripRows hold
+// the full prefix, the others the prefix within their strip.
+constexpr int kStripRows = 8;
+__device__ __forceinline__ long long table_at(const long long* t, int stride, int y, int x) {
+    const long long v = t[(size_t)y * stride + x];
+    return y % kStripRows ? v + t[(size_t)(y / kStripRows * kStripRows) * stride + x] : v;
+}
+
 // IntegralImage::stats (preprocess.rs:114-125) from exact sums: mean and standard deviation as
 // the reference's f64 arithmetic would round them to f32.
 __device__ __forceinline__ void fix_stats(long long sum1, long long sum2, const FixScale& fs, float count,

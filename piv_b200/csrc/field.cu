@@ -53,7 +53,11 @@ __device__ __forceinline__ float2 place1(int origin, float shift, float mx) {
     return make_float2(a0, __fadd_rn(a0, s));
 }
 
-__device__ __forceinline__ long long rect(const long long* t, int stride, int x0, int y0, int x1, int y1) {
+__device__ __forceinline__ long long rect(const StatsView& s, const long long* t, int x0, int y0, int x1, int y1) {
+    const int stride = s.W + 1;
+    if (s.strips)
+        return table_at(t, stride, y1, x1) - table_at(t, stride, y0, x1) - table_at(t, stride, y1, x0) +
+               table_at(t, stride, y0, x0);
     return t[(size_t)y1 * stride + x1] - t[(size_t)y0 * stride + x1] - t[(size_t)y1 * stride + x0] + t[(size_t)y0 * stride + x0];
 }
 
@@ -62,11 +66,10 @@ __device__ bool has_signal(const StatsView& s, float x, float y, int n, float mi
     int bx = (int)roundf(x), by = (int)roundf(y);  // f32::round: half away from zero
     bx = min(max(bx, 0), s.W - n);
     by = min(max(by, 0), s.H - n);
-    const int stride = s.W + 1;
     const FixScale fs{s.scales[0], s.scales[1]};
     float mean, sd;
-    fix_stats(rect(s.sum, stride, bx, by, bx + n, by + n), rect(s.sumsq, stride, bx, by, bx + n, by + n), fs,
-              (float)(n * n), &mean, &sd);
+    fix_stats(rect(s, s.sum, bx, by, bx + n, by + n), rect(s, s.sumsq, bx, by, bx + n, by + n), fs, (float)(n * n), &mean,
+              &sd);
     return mean >= min_mean && sd >= min_std;
 }
 

@@ -91,6 +91,7 @@ struct StatsView {
     const long long* sumsq;  // (H+1) x (W+1)
     const int* scales;       // [s1, s2]
     int H, W;
+    int strips;  // 1: tables stored in strips (table_at), 0: plain prefixes (a caller's own tables)
 };
 
 struct PlaceParams {
@@ -183,17 +184,17 @@ struct PrepParams {
     long long* sum;
     long long* sumsq;
     int* scales;
-    unsigned int* maxbits;    // scratch word
+    unsigned int* maxbits;    // 2 scratch words: max |base|, max |blurred|
 };
 
 // Runs the whole PreparedFrame::new chain; returns the number of kernels launched in *launches.
 cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches);
-// Integral tables only (used when the prepared image is supplied directly).
 // The reference's f64 IntegralImage tables, already copied into `sum` / `sumsq` (8 bytes per
-// entry, (H+1) x (W+1)), converted in place to the fixed-point tables launch_stats builds;
+// entry, (H+1) x (W+1)), converted in place to plain fixed-point tables;
 // *nonfinite becomes nonzero if an entry is not finite. maxbits2: 2 device words of scratch.
 cudaError_t launch_tables_to_fixed(long long* sum, long long* sumsq, int H, int W, int* scales,
                                    unsigned long long* maxbits2, unsigned int* nonfinite, cudaStream_t s, int* launches);
+// Integral tables only (used when the prepared image is supplied directly), stored in strips.
 cudaError_t launch_stats(const float* base, int H, int W, long long* sum, long long* sumsq, int* scales,
                          unsigned int* maxbits, cudaStream_t s, int* launches);
 

@@ -135,17 +135,47 @@ struct FloatSamples {
     }
 };
 
+// ------------------------------------------------------------------------------- max |v|
+// Folds each thread's running max |v| into *out: one atomic per block of <= 256 threads. Every
+// thread of the block calls it.
+__device__ __forceinline__ void block_max_to(float m, unsigned int* out) {
+    __shared__ float wmax[8];
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = threadIdx.x < (blockDim.x >> 5) ? wmax[threadIdx.x] : 0.0f;
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (threadIdx.x == 0) atomicMax(out, __float_as_uint(m));  // non-negative floats order as uints
+    }
+}
+
+__global__ void maxabs_kernel(const float* __restrict__ v, long long n, unsigned int* out) {
+    float m = 0.0f;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        m = fmaxf(m, fabsf(v[i]));
+    block_max_to(m, out);
+}
+
+// ------------------------------------------------------------------------------- conversion kernels
 // Streams codes 16 bytes per load (8 u16 or 16 u8) when the buffers are 16-byte aligned; the
-// rest of the frame (or an unaligned one) one code at a time.
+// rest of the frame (or an unaligned one) one code at a time. With a non-null `maxout` the kernel
+// also folds max |value| into it (the scale of the fixed-point sums), which saves a pass over the
+// frame. Launched with 256 threads.
 template <typename CodeT>
 __global__ void convert_kernel(const CodeT* __restrict__ raw, long long n, const float* __restrict__ bg,
-                               const unsigned int* clip, float* __restrict__ out) {
+                               const unsigned int* clip, float* __restrict__ out, unsigned int* maxout) {
     constexpr int V = 16 / (int)sizeof(CodeT);
     CodeSamples<CodeT> src{raw, bg, clip, 0u, 0.0f, 0.0f};
     src.begin();
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
-    auto value = [&](unsigned int c, float b) { return src.value(c, b); };
+    float m = 0.0f;
+    auto value = [&](unsigned int c, float b) {
+        const float v = src.value(c, b);
+        m = fmaxf(m, fabsf(v));
+        return v;
+    };
     long long head = 0;
     const bool aligned = (reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(out) |
                           reinterpret_cast<uintptr_t>(bg)) % 16 == 0;
@@ -172,143 +202,128 @@ __global__ void convert_kernel(const CodeT* __restrict__ raw, long long n, const
         head = nv * V;
     }
     for (long long i = head + tid; i < n; i += stride) out[i] = value(raw[i], bg ? bg[i] : 0.0f);
+    if (maxout) block_max_to(m, maxout);
 }
 
 __global__ void convert_f32_kernel(const float* __restrict__ raw, long long n, const float* __restrict__ bg,
-                                   float* __restrict__ out) {
+                                   float* __restrict__ out, unsigned int* maxout) {
     const FloatSamples src{raw, bg};
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        out[i] = src((size_t)i);
-}
-
-// ------------------------------------------------------------------------------- max |v|
-// One atomic per block (the block's warps reduce through shared memory first); launched with
-// 256 threads.
-// Folds each thread's running max |v| into *out: one atomic per block of <= 256 threads. Every
-// thread of the block calls it.
-__device__ __forceinline__ void block_max_to(float m, unsigned int* out) {
-    __shared__ float wmax[8];
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        m = threadIdx.x < (blockDim.x >> 5) ? wmax[threadIdx.x] : 0.0f;
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (threadIdx.x == 0) atomicMax(out, __float_as_uint(m));  // non-negative floats order as uints
-    }
-}
-
-__global__ void maxabs_kernel(const float* __restrict__ v, long long n, unsigned int* out) {
     float m = 0.0f;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        m = fmaxf(m, fabsf(v[i]));
-    block_max_to(m, out);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const float v = src((size_t)i);
+        m = fmaxf(m, fabsf(v));
+        out[i] = v;
+    }
+    if (maxout) block_max_to(m, maxout);
 }
 
 // ------------------------------------------------------------------------------- integral tables
-// Row pass: T[y+1][x+1] = sum_{x' <= x} q(v[y][x']) for both tables; T[y+1][0] = 0.
-__global__ void integral_rows_kernel(const float* __restrict__ v, int H, int W, long long* sum, long long* sumsq,
-                                     const unsigned int* maxbits, int* scales) {
-    const int y = blockIdx.x;
+// T[y][x] = sum of q(v) over the rows above y and the columns left of x, for q = value and square,
+// in strips of kStripRows rows: the strip kernel writes each strip's own 2-D prefix (one block per
+// strip, every pixel read once), and the scan kernel turns every kStripRows-th row into the full
+// prefix, in place. A reader adds the full row above an entry's strip (table_at in common.cuh), so
+// no third pass over the tables is needed. Integer sums: any order gives the same bits.
+//
+// Writing 16 bytes per pixel bounds both tables. Two passes over all rows (a running sum down every
+// column, W / 128 blocks) left most SMs without a block and took 236 us of a 1437 x 1003 frame's
+// 310 us preparation; a masked pair of that size went from 667 to 394 us in all (B200).
+constexpr int kStripThreads = 512;
+constexpr int kStripWarps = kStripThreads / 32;
+
+__device__ __forceinline__ long long warp_scan(long long v, int lane) {
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    return v;
+}
+
+__global__ void __launch_bounds__(kStripThreads) integral_strip_kernel(const float* __restrict__ v, int H, int W,
+                                                                       long long* __restrict__ sum,
+                                                                       long long* __restrict__ sumsq,
+                                                                       const unsigned int* maxbits, int* scales) {
+    constexpr int R = kStripRows;
+    static_assert(2 * R == kStripWarps, "one warp scans the warp totals of each row of each table");
     const FixScale fs = fix_scale(__uint_as_float(*maxbits), (long long)H * W);
-    if (y == 0 && threadIdx.x == 0) {
-        scales[0] = fs.s1;
-        scales[1] = fs.s2;
-    }
+    const int y0 = blockIdx.x * R, rows = min(R, H - y0);
     const int stride = W + 1;
-    long long* r1 = sum + (size_t)(y + 1) * stride;
-    long long* r2 = sumsq + (size_t)(y + 1) * stride;
-    const float* row = v + (size_t)y * W;
-    __shared__ long long c1[32], c2[32];
-    __shared__ long long carry1, carry2;
-    if (threadIdx.x == 0) {
-        r1[0] = 0;
-        r2[0] = 0;
-        carry1 = 0;
-        carry2 = 0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ long long tot[kStripWarps][2 * R + 1];  // [warp][row of table 1, row of table 2]
+    if (blockIdx.x == 0) {
+        if (tid == 0) {
+            scales[0] = fs.s1;
+            scales[1] = fs.s2;
+        }
+        for (int x = tid; x <= W; x += kStripThreads) sum[x] = sumsq[x] = 0;
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int base = 0; base < W; base += blockDim.x) {
-        const int x = base + threadIdx.x;
-        long long a = 0, b = 0;
-        if (x < W) {
-            const float f = row[x];
-            a = fix_q1(f, fs);
-            b = fix_q2(f, fs);
+    if (tid < 2 * rows) (tid < rows ? sum : sumsq)[(size_t)(y0 + 1 + tid % rows) * stride] = 0;
+    long long carry = 0;  // warp j: total of value row j over the columns before `base`
+    for (int base = 0; base < W; base += kStripThreads) {
+        const int x = base + tid;
+        long long a[R], b[R];  // running sums down the column, then 2-D prefixes within the warp
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float f = (x < W && r < rows) ? v[(size_t)(y0 + r) * W + x] : 0.0f;
+            a[r] = fix_q1(f, fs) + (r ? a[r - 1] : 0);
+            b[r] = fix_q2(f, fs) + (r ? b[r - 1] : 0);
         }
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long ua = __shfl_up_sync(0xffffffffu, a, o), ub = __shfl_up_sync(0xffffffffu, b, o);
-            if (lane >= o) {
-                a += ua;
-                b += ub;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            a[r] = warp_scan(a[r], lane);
+            b[r] = warp_scan(b[r], lane);
+            if (lane == 31) {
+                tot[warp][r] = a[r];
+                tot[warp][R + r] = b[r];
             }
         }
-        if (lane == 31) {
-            c1[warp] = a;
-            c2[warp] = b;
+        __syncthreads();
+        {
+            const long long t = lane < kStripWarps ? tot[lane][warp] : 0;
+            const long long incl = warp_scan(t, lane);
+            if (lane < kStripWarps) tot[lane][warp] = carry + incl - t;
+            carry += __shfl_sync(0xffffffffu, incl, 31);
         }
         __syncthreads();
-        if (warp == 0) {
-            long long wa = lane < nw ? c1[lane] : 0, wb = lane < nw ? c2[lane] : 0;
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long ua = __shfl_up_sync(0xffffffffu, wa, o), ub = __shfl_up_sync(0xffffffffu, wb, o);
-                if (lane >= o) {
-                    wa += ua;
-                    wb += ub;
+        if (x < W) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r < rows) {
+                    const size_t o = (size_t)(y0 + 1 + r) * stride + x + 1;
+                    sum[o] = a[r] + tot[warp][r];
+                    sumsq[o] = b[r] + tot[warp][R + r];
                 }
-            }
-            if (lane < nw) {
-                c1[lane] = wa;
-                c2[lane] = wb;
-            }
-        }
-        __syncthreads();
-        const long long off1 = carry1 + (warp > 0 ? c1[warp - 1] : 0);
-        const long long off2 = carry2 + (warp > 0 ? c2[warp - 1] : 0);
-        if (x < W) {
-            r1[x + 1] = a + off1;
-            r2[x + 1] = b + off2;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            carry1 += c1[nw - 1];
-            carry2 += c2[nw - 1];
         }
         __syncthreads();
     }
 }
 
-// Column pass: cumulative sums down each column of both tables (rows 1..H). Row 0 is zero.
-__global__ void integral_cols_kernel(int H, int W, long long* sum, long long* sumsq) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+// Rows kStripRows, 2 kStripRows, ... of both tables become running sums down each column: 32
+// columns and 32 groups of strips per block.
+__global__ void __launch_bounds__(1024) integral_scan_kernel(int H, int W, long long* sum, long long* sumsq) {
+    const int strips = H / kStripRows;  // full strips; a last partial one has no row to update
     const int stride = W + 1;
-    if (x > W) return;
-    sum[x] = 0;
-    sumsq[x] = 0;
-    long long a = 0, b = 0;
-    int y = 1;
-    for (; y + 4 <= H + 1; y += 4) {
-        long long va[4], vb[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            va[i] = sum[(size_t)(y + i) * stride + x];
-            vb[i] = sumsq[(size_t)(y + i) * stride + x];
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            a += va[i];
-            b += vb[i];
-            sum[(size_t)(y + i) * stride + x] = a;
-            sumsq[(size_t)(y + i) * stride + x] = b;
-        }
+    const int tx = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int x = blockIdx.x * 32 + tx;
+    const int per = (strips + 31) / 32, s0 = min(g * per, strips), s1 = min(s0 + per, strips);
+    __shared__ long long part[2][32][32];
+    long long* const t[2] = {sum, sumsq};
+    long long acc[2] = {0, 0};
+    if (x <= W)
+        for (int s = s0; s < s1; ++s)
+            for (int k = 0; k < 2; ++k) acc[k] += t[k][(size_t)(s + 1) * kStripRows * stride + x];
+    for (int k = 0; k < 2; ++k) part[k][g][tx] = acc[k];
+    __syncthreads();
+    for (int k = 0; k < 2; ++k) {
+        acc[k] = 0;
+        for (int j = 0; j < g; ++j) acc[k] += part[k][j][tx];
     }
-    for (; y <= H; ++y) {
-        a += sum[(size_t)y * stride + x];
-        b += sumsq[(size_t)y * stride + x];
-        sum[(size_t)y * stride + x] = a;
-        sumsq[(size_t)y * stride + x] = b;
-    }
+    if (x <= W)
+        for (int s = s0; s < s1; ++s)
+            for (int k = 0; k < 2; ++k) {
+                long long* e = t[k] + (size_t)(s + 1) * kStripRows * stride + x;
+                acc[k] += *e;
+                *e = acc[k];
+            }
 }
 
 // ------------------------------------------------------------------------------- blur
@@ -565,16 +580,23 @@ __global__ void table_to_fixed_kernel(unsigned long long* t, long long n, const 
         t[i] = (unsigned long long)f64_bits_to_fixed(t[i], s);
 }
 
+// The tables from `base` and its max |v| in *maxbits.
+static cudaError_t run_tables(const float* base, int H, int W, long long* sum, long long* sumsq, int* scales,
+                              const unsigned int* maxbits, cudaStream_t s, int* launches) {
+    integral_strip_kernel<<<(H + kStripRows - 1) / kStripRows, kStripThreads, 0, s>>>(base, H, W, sum, sumsq, maxbits, scales);
+    integral_scan_kernel<<<(W + 1 + 31) / 32, 1024, 0, s>>>(H, W, sum, sumsq);
+    if (launches) *launches += 2;
+    return cudaGetLastError();
+}
+
 cudaError_t launch_stats(const float* base, int H, int W, long long* sum, long long* sumsq, int* scales,
                          unsigned int* maxbits, cudaStream_t s, int* launches) {
     const long long n = (long long)H * W;
     cudaError_t e = cudaMemsetAsync(maxbits, 0, sizeof(unsigned int), s);
     if (e != cudaSuccess) return e;
     maxabs_kernel<<<grid_for(n), 256, 0, s>>>(base, n, maxbits);
-    integral_rows_kernel<<<H, 256, 0, s>>>(base, H, W, sum, sumsq, maxbits, scales);
-    integral_cols_kernel<<<(W + 1 + 127) / 128, 128, 0, s>>>(H, W, sum, sumsq);
-    if (launches) *launches += 3;
-    return cudaGetLastError();
+    if (launches) *launches += 1;
+    return run_tables(base, H, W, sum, sumsq, scales, maxbits, s, launches);
 }
 
 // Blur weights exactly as preprocess.rs:162-168 computes them (f32 exp of an f32 argument,
@@ -642,20 +664,28 @@ cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches) {
     // integral tables are wanted, the blur decodes the raw samples itself and base is not written.
     float* base = p.base;
     const bool fused = blur && !p.build_stats;
+    // max |base| for the tables' scale, and for the normalisation's when it reads base itself: both
+    // find it in words the conversion fills.
+    const bool base_max = p.build_stats || (norm && !blur);
+    if (base_max || norm) {
+        e = cudaMemsetAsync(p.maxbits, 0, 2 * sizeof(unsigned int), s);
+        if (e != cudaSuccess) return e;
+    }
+    unsigned int* bmax = base_max ? p.maxbits : nullptr;
     if (!fused) switch (p.raw_type) {
         case RAW_U8:
-            convert_kernel<uint8_t><<<grid_for(n), 256, 0, s>>>((const uint8_t*)p.raw, n, p.background, clip, base);
+            convert_kernel<uint8_t><<<grid_for(n), 256, 0, s>>>((const uint8_t*)p.raw, n, p.background, clip, base, bmax);
             break;
         case RAW_U16:
-            convert_kernel<uint16_t><<<grid_for(n), 256, 0, s>>>((const uint16_t*)p.raw, n, p.background, clip, base);
+            convert_kernel<uint16_t><<<grid_for(n), 256, 0, s>>>((const uint16_t*)p.raw, n, p.background, clip, base, bmax);
             break;
         default:
-            convert_f32_kernel<<<grid_for(n), 256, 0, s>>>((const float*)p.raw, n, p.background, base);
+            convert_f32_kernel<<<grid_for(n), 256, 0, s>>>((const float*)p.raw, n, p.background, base, bmax);
             break;
     }
     if (!fused) nl += 1;
     if (p.build_stats) {
-        e = launch_stats(base, p.H, p.W, p.sum, p.sumsq, p.scales, p.maxbits, s, &nl);
+        e = run_tables(base, p.H, p.W, p.sum, p.sumsq, p.scales, p.maxbits, s, &nl);
         if (e != cudaSuccess) return e;
     }
     const float* cur = base;
@@ -666,10 +696,6 @@ cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches) {
         const size_t sm = sizeof(float) * ((size_t)(BT_Y + 2 * R) * (BT_X + 2 * R) + (size_t)(BT_Y + 2 * R) * BT_X);
         float* dst = norm ? p.tmp : p.image;
         unsigned int* mx = norm ? p.maxbits + 1 : nullptr;
-        if (norm) {
-            e = cudaMemsetAsync(mx, 0, sizeof(unsigned int), s);
-            if (e != cudaSuccess) return e;
-        }
         dim3 grid((p.W + BT_X - 1) / BT_X, (p.H + BT_Y - 1) / BT_Y);
         if (!fused) {
             e = run_blur(grid, sm, s, FloatSamples{cur, nullptr}, p.H, p.W, k, dst, mx);
@@ -689,22 +715,17 @@ cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches) {
     if (norm) {
         const int r = p.normalize_radius;
         if (r > kMaxNormRadius) return cudaErrorInvalidValue;
-        if (!blur) {
-            e = cudaMemsetAsync(p.maxbits + 1, 0, sizeof(unsigned int), s);
-            if (e != cudaSuccess) return e;
-            maxabs_kernel<<<grid_for(n), 256, 0, s>>>(cur, n, p.maxbits + 1);
-            nl += 1;
-        }
+        const unsigned int* const mx = blur ? p.maxbits + 1 : p.maxbits;  // max |cur|
         const size_t sm = sizeof(long long) * (2 * (size_t)(NT_Y + 2 * r) * ((NT_X + 2 * r) | 1) + 2 * (size_t)(NT_Y + 2 * r) * NT_HW);
         dim3 grid((p.W + NT_X - 1) / NT_X, (p.H + NT_Y - 1) / NT_Y);
         if (r == 4) {  // the default radius: 46.3 KB of tile, under the 48 KB default
-            normalize_kernel<4><<<grid, kNormThreads, sm, s>>>(cur, p.H, p.W, r, p.normalize_eps, p.maxbits + 1, p.image);
+            normalize_kernel<4><<<grid, kNormThreads, sm, s>>>(cur, p.H, p.W, r, p.normalize_eps, mx, p.image);
         } else {
             if (sm > 48 * 1024) {
                 e = cudaFuncSetAttribute(normalize_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
                 if (e != cudaSuccess) return e;
             }
-            normalize_kernel<0><<<grid, kNormThreads, sm, s>>>(cur, p.H, p.W, r, p.normalize_eps, p.maxbits + 1, p.image);
+            normalize_kernel<0><<<grid, kNormThreads, sm, s>>>(cur, p.H, p.W, r, p.normalize_eps, mx, p.image);
         }
         nl += 1;
         cur = p.image;
