@@ -484,11 +484,8 @@ int32_t piv_tc_wait_probe(int32_t device, int32_t log2_iters, int32_t* timed_out
  * acquisition loops (cudaFree waits for the whole device) and processes whose device memory is
  * already reserved by another allocator. All pointers are DEVICE pointers owned by the caller;
  * work is queued on `stream` (NULL = the default stream) and the call returns without waiting.
- * Scratch lives in a fixed device array inside the library of 2 x 2,097,152 bytes, held by every
- * GPU that loads the library until exit; fields above 2,097,152 cells are rejected
- * (PIV_ERR_UNSUPPORTED). The first call on a device looks up that array's address, so make it
- * before any stream capture; the address is kept until exit, so do not call this on a device
- * after cudaDeviceReset. All calls share the array: calls whose work overlaps on the GPU race.
+ * Fields above 2,097,152 cells are rejected (PIV_ERR_UNSUPPORTED). The kernel keeps its flag
+ * snapshots in shared memory, so calls share nothing and may overlap on the GPU.
  * Outputs must not overlap any input or each other (the median test reads neighbours while
  * others are written): such calls are rejected (PIV_ERR_ARGUMENT). */
 int32_t piv_validate_field_noalloc(int64_t ny, int64_t nx, const float* dx, const float* dy, const float* peak_ratio,

@@ -80,8 +80,6 @@ struct PassBuf {
     float* raw_dy;
     float* raw_ppr;
     uint8_t* raw_flags;
-    uint8_t* f1;
-    uint8_t* f2;
     float* dx;
     float* dy;
     uint8_t* flags;
@@ -226,7 +224,7 @@ int use_device(PivAnalyzer* an) {
 }
 
 // Per-pair workspace for up to K pairs of (H, W) frames: for every pass, origins, signal status,
-// raw field, two flag snapshots and the validated field; 8 summary counters per pair.
+// raw field and the validated field; 8 summary counters per pair.
 int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
     if (an->arena && an->H == H && an->W == W && an->K >= K) return PIV_OK;
     if (an->arena) {
@@ -245,7 +243,7 @@ int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
         pb.cells = pb.grid.nx * pb.grid.ny;
         if (pb.cells > (int64_t)1 << 30) return fail(PIV_ERR_UNSUPPORTED, "too many windows in one pass");
         const size_t c = (size_t)pb.cells;
-        per_pair += align256(16 * c) + align256(c) + 3 * align256(4 * c) + 3 * align256(c) + 2 * align256(4 * c) + align256(c) +
+        per_pair += align256(16 * c) + align256(c) + 3 * align256(4 * c) + align256(c) + 2 * align256(4 * c) + align256(c) +
                     (an->deform ? align256(32 * c) : 0);
         proto.push_back(pb);
     }
@@ -268,8 +266,6 @@ int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
             pb.raw_dy = (float*)take(4 * c);
             pb.raw_ppr = (float*)take(4 * c);
             pb.raw_flags = (uint8_t*)take(c);
-            pb.f1 = (uint8_t*)take(c);
-            pb.f2 = (uint8_t*)take(c);
             pb.dx = (float*)take(4 * c);
             pb.dy = (float*)take(4 * c);
             pb.flags = (uint8_t*)take(c);
@@ -348,12 +344,14 @@ int run_passes_eager(PivAnalyzer* an, const PivFrame* const* a, const PivFrame* 
             }
             pp.min_mean = an->min_mean;
             pp.min_std = an->min_std;
+            pp.zero_counts = i == 0 ? an->d_counts + 8 * (size_t)k : nullptr;
             cps[k] = CorrParams{a[k]->image, b[k]->image, (int)H, (int)W, pb.origins, pb.status, (int)pb.cells,
                                 pb.raw_dx, pb.raw_dy, pb.raw_ppr, pb.raw_flags, pp.corners, (int)pb.grid.x0,
                                 (int)pb.grid.y0, (int)pb.grid.step, (int)pb.grid.nx};
             vps[k] = ValidateParams{(int)pb.grid.nx, (int)pb.grid.ny, pb.raw_dx, pb.raw_dy, pb.raw_ppr, pb.raw_flags,
-                                    pb.f1, pb.f2, pb.dx, pb.dy, pb.flags, (float)an->windows[0] / 2.0f,
-                                    an->ppr_threshold, an->median_threshold, an->median_eps, an->replace};
+                                    pb.dx, pb.dy, pb.flags, (float)an->windows[0] / 2.0f, an->ppr_threshold,
+                                    an->median_threshold, an->median_eps, an->replace,
+                                    i + 1 == npass ? an->d_counts + 8 * (size_t)k : nullptr};
         }
         int nl = 0;
         CUDA_TRY(launch_place_items(pps.data(), K, an->cur, &nl));
@@ -424,14 +422,6 @@ int run_passes_eager(PivAnalyzer* an, const PivFrame* const* a, const PivFrame* 
         CUDA_TRY(launch_validate_items(vps.data(), K, an->cur, &nl));
         an->launches += nl;
     }
-    std::vector<SummaryItem> sums(K);
-    for (int k = 0; k < K; ++k) {
-        const PassBuf& last = an->pairs[k].back();
-        sums[k] = SummaryItem{last.flags, (int)last.cells, an->d_counts + 8 * (size_t)k};
-    }
-    int nl = 0;
-    CUDA_TRY(launch_summary_items(sums.data(), K, an->cur, &nl));
-    an->launches += nl;
     return PIV_OK;
 }
 
@@ -932,20 +922,65 @@ int32_t piv_background_device(PivAnalyzer* an, const void* frames_dev, int32_t d
     return PIV_OK;
 }
 
+namespace {
+
+// Whether a kernel on `dev` can write all of these buffers directly (null ones are skipped). Other
+// memory (another device's, unregistered host memory) keeps the copy commands.
+bool kernel_writable(int dev, std::initializer_list<const void*> ptrs) {
+    for (const void* p : ptrs) {
+        if (!p) continue;
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type == cudaMemoryTypeUnregistered || (at.type == cudaMemoryTypeDevice && at.device != dev)) return false;
+    }
+    return true;
+}
+
+// The final fields of the workspace's first `count` pairs, one after another, into the caller's
+// buffers on the analyzer's stream; `counts_out` has `count_stride` counters per pair.
+int export_fields(PivAnalyzer* an, int count, float* dx, float* dy, float* peak_ratio, uint8_t* flags,
+                  unsigned long long* counts_out, int count_stride) {
+    const size_t c = (size_t)an->pairs[0].back().cells;
+    if (kernel_writable(an->device, {dx, dy, peak_ratio, flags, counts_out})) {
+        std::vector<ExportItem> items(count);
+        for (int k = 0; k < count; ++k) {
+            const PassBuf& last = an->pairs[k].back();
+            const size_t o = k * c;
+            items[k] = ExportItem{last.dx, last.dy, last.raw_ppr, last.flags, an->d_counts + 8 * (size_t)k, (int)c,
+                                  dx ? dx + o : nullptr, dy ? dy + o : nullptr, peak_ratio ? peak_ratio + o : nullptr,
+                                  flags ? flags + o : nullptr,
+                                  counts_out ? counts_out + (size_t)count_stride * k : nullptr};
+        }
+        int nl = 0;
+        CUDA_TRY(launch_export_items(items.data(), count, an->cur, &nl));
+        an->launches += nl;
+        return PIV_OK;
+    }
+    for (int k = 0; k < count; ++k) {
+        const PassBuf& last = an->pairs[k].back();
+        const size_t o = k * c;
+        if (dx) CUDA_TRY(cudaMemcpyAsync(dx + o, last.dx, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
+        if (dy) CUDA_TRY(cudaMemcpyAsync(dy + o, last.dy, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
+        if (peak_ratio) CUDA_TRY(cudaMemcpyAsync(peak_ratio + o, last.raw_ppr, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
+        if (flags) CUDA_TRY(cudaMemcpyAsync(flags + o, last.flags, c, cudaMemcpyDeviceToDevice, an->cur));
+        if (counts_out)
+            CUDA_TRY(cudaMemcpyAsync(counts_out + (size_t)count_stride * k, an->d_counts + 8 * (size_t)k,
+                                     5 * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, an->cur));
+    }
+    return PIV_OK;
+}
+
+}  // namespace
+
 int32_t piv_analyze_device(PivAnalyzer* an, const PivFrame* a, const PivFrame* b, float* dx, float* dy,
                            float* peak_ratio, uint8_t* flags, uint64_t* summary_dev) {
     if (!an) return fail(PIV_ERR_ARGUMENT, "null analyzer");
     int st = run_passes(an, a, b);
     if (st) return st;
-    const PassBuf& last = an->pairs[0].back();
-    const size_t c = (size_t)last.cells;
-    if (dx) CUDA_TRY(cudaMemcpyAsync(dx, last.dx, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
-    if (dy) CUDA_TRY(cudaMemcpyAsync(dy, last.dy, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
-    if (peak_ratio) CUDA_TRY(cudaMemcpyAsync(peak_ratio, last.raw_ppr, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
-    if (flags) CUDA_TRY(cudaMemcpyAsync(flags, last.flags, c, cudaMemcpyDeviceToDevice, an->cur));
-    if (summary_dev)
-        CUDA_TRY(cudaMemcpyAsync(summary_dev, an->d_counts, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, an->cur));
-    return PIV_OK;
+    return export_fields(an, 1, dx, dy, peak_ratio, flags, (unsigned long long*)summary_dev, 5);
 }
 
 int32_t piv_analyze(PivAnalyzer* an, const PivFrame* a, const PivFrame* b, float* dx, float* dy, float* peak_ratio,
@@ -1286,7 +1321,7 @@ int32_t piv_validate_field(PivAnalyzer* an, int64_t ny, int64_t nx, const float*
     if (st) return st;
     const size_t c = (size_t)(ny * nx);
     void* buf = nullptr;
-    CUDA_TRY(cudaMalloc(&buf, 5 * align256(4 * c) + 4 * align256(c) + 256));
+    CUDA_TRY(cudaMalloc(&buf, 5 * align256(4 * c) + 2 * align256(c) + 256));
     char* p = (char*)buf;
     auto take = [&](size_t bytes) {
         void* r = p;
@@ -1299,19 +1334,17 @@ int32_t piv_validate_field(PivAnalyzer* an, int64_t ny, int64_t nx, const float*
     float* o_dx = (float*)take(4 * c);
     float* o_dy = (float*)take(4 * c);
     uint8_t* f0 = (uint8_t*)take(c);
-    uint8_t* f1 = (uint8_t*)take(c);
-    uint8_t* f2 = (uint8_t*)take(c);
     uint8_t* fo = (uint8_t*)take(c);
     unsigned long long* cnt = (unsigned long long*)take(64);
     cudaError_t e = cudaMemcpyAsync(d_dx, dx, 4 * c, cudaMemcpyHostToDevice, an->cur);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_dy, dy, 4 * c, cudaMemcpyHostToDevice, an->cur);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_ppr, peak_ratio, 4 * c, cudaMemcpyHostToDevice, an->cur);
     if (e == cudaSuccess) e = cudaMemcpyAsync(f0, flags, c, cudaMemcpyHostToDevice, an->cur);
-    ValidateParams vp{(int)nx, (int)ny, d_dx, d_dy, d_ppr, f0, f1, f2, o_dx, o_dy, fo, (float)an->windows[0] / 2.0f,
-                      an->ppr_threshold, an->median_threshold, an->median_eps, an->replace};
+    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, 64, an->cur);
+    ValidateParams vp{(int)nx, (int)ny, d_dx, d_dy, d_ppr, f0, o_dx, o_dy, fo, (float)an->windows[0] / 2.0f,
+                      an->ppr_threshold, an->median_threshold, an->median_eps, an->replace, cnt};
     if (e == cudaSuccess) e = launch_validate(vp, an->cur);
-    if (e == cudaSuccess) e = launch_summary(fo, (int)c, cnt, an->cur);
-    an->launches += kValidateLaunches + kSummaryLaunches;
+    an->launches += kValidateLaunches;
     unsigned long long hc[5] = {0, 0, 0, 0, 0};
     if (e == cudaSuccess && out_dx) e = cudaMemcpyAsync(out_dx, o_dx, 4 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && out_dy) e = cudaMemcpyAsync(out_dy, o_dy, 4 * c, cudaMemcpyDeviceToHost, an->cur);
@@ -1335,18 +1368,7 @@ int32_t piv_analyze_batch_device(PivAnalyzer* an, const PivFrame* const* a, cons
     if (!an || !a || !b) return fail(PIV_ERR_ARGUMENT, "null argument");
     int st = run_passes(an, a, b, count);
     if (st) return st;
-    for (int k = 0; k < count; ++k) {
-        const PassBuf& last = an->pairs[k].back();
-        const size_t c = (size_t)last.cells;
-        if (dx) CUDA_TRY(cudaMemcpyAsync(dx + k * c, last.dx, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
-        if (dy) CUDA_TRY(cudaMemcpyAsync(dy + k * c, last.dy, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
-        if (peak_ratio) CUDA_TRY(cudaMemcpyAsync(peak_ratio + k * c, last.raw_ppr, 4 * c, cudaMemcpyDeviceToDevice, an->cur));
-        if (flags) CUDA_TRY(cudaMemcpyAsync(flags + k * c, last.flags, c, cudaMemcpyDeviceToDevice, an->cur));
-    }
-    if (summaries_dev)
-        CUDA_TRY(cudaMemcpyAsync(summaries_dev, an->d_counts, 8 * sizeof(unsigned long long) * (size_t)count,
-                                 cudaMemcpyDeviceToDevice, an->cur));
-    return PIV_OK;
+    return export_fields(an, count, dx, dy, peak_ratio, flags, (unsigned long long*)summaries_dev, 8);
 }
 
 namespace {
@@ -1887,7 +1909,7 @@ size_t request_bytes(const Request& r, bool stats, bool chain, bool both, size_t
     b += 2 * align256(4 * (4 + 512 + 4)) + 2 * align256(8);
     for (const PassBuf& pb : r.passes) {
         const size_t c = (size_t)pb.cells;
-        b += align256(16 * c) + align256(c) + 3 * align256(4 * c) + 3 * align256(c) + 2 * align256(4 * c) + align256(c) +
+        b += align256(16 * c) + align256(c) + 3 * align256(4 * c) + align256(c) + 2 * align256(4 * c) + align256(c) +
              (r.cfg.deform ? align256(32 * c) : 0);
     }
     return b + align256(8 * sizeof(unsigned long long));
@@ -1999,8 +2021,6 @@ int admit_request(PivServer* sv, Request* r, bool inject_failure) {
         pb.raw_dy = (float*)take(4 * c);
         pb.raw_ppr = (float*)take(4 * c);
         pb.raw_flags = (uint8_t*)take(c);
-        pb.f1 = (uint8_t*)take(c);
-        pb.f2 = (uint8_t*)take(c);
         pb.dx = (float*)take(4 * c);
         pb.dy = (float*)take(4 * c);
         pb.flags = (uint8_t*)take(c);
@@ -2125,6 +2145,7 @@ void PivServer::launch_step(std::vector<Request*>& work) {
         }
         pp.min_mean = r->cfg.min_mean;
         pp.min_std = r->cfg.min_std;
+        pp.zero_counts = i == 0 ? r->d_counts : nullptr;
         pps.push_back(pp);
         // 0 / 1: FP32 uniform / deformed windows; 2 / 3: tensor cores, BF16 / FP16 split, uniform;
         // 4 / 5: the same with deformed windows
@@ -2135,9 +2156,10 @@ void PivServer::launch_step(std::vector<Request*>& work) {
             CorrParams{r->fa.image, r->fb.image, (int)r->H, (int)r->W, pb.origins, pb.status, (int)pb.cells, pb.raw_dx,
                        pb.raw_dy, pb.raw_ppr, pb.raw_flags, pp.corners, (int)pb.grid.x0, (int)pb.grid.y0,
                        (int)pb.grid.step, (int)pb.grid.nx});
-        vps.push_back(ValidateParams{(int)pb.grid.nx, (int)pb.grid.ny, pb.raw_dx, pb.raw_dy, pb.raw_ppr, pb.raw_flags, pb.f1,
-                                     pb.f2, pb.dx, pb.dy, pb.flags, (float)r->cfg.windows[0] / 2.0f, r->cfg.ppr_threshold,
-                                     r->cfg.median_threshold, r->cfg.median_eps, r->cfg.replace});
+        vps.push_back(ValidateParams{(int)pb.grid.nx, (int)pb.grid.ny, pb.raw_dx, pb.raw_dy, pb.raw_ppr, pb.raw_flags, pb.dx,
+                                     pb.dy, pb.flags, (float)r->cfg.windows[0] / 2.0f, r->cfg.ppr_threshold,
+                                     r->cfg.median_threshold, r->cfg.median_eps, r->cfg.replace,
+                                     i + 1 == (int)r->passes.size() ? r->d_counts : nullptr});
     }
     int nl = 0;
     cudaError_t e = launch_place_items(pps.data(), (int)pps.size(), stream, &nl);
@@ -2166,17 +2188,13 @@ void PivServer::launch_step(std::vector<Request*>& work) {
                     : launch_correlate_items(kv.first.first, variant[kv.first.second][kv.first.first], kv.second.data(),
                                              (int)kv.second.size(), stream, &nl);
     if (e == cudaSuccess) e = launch_validate_items(vps.data(), (int)vps.size(), stream, &nl);
-    std::vector<SummaryItem> sums;
+    bool finished = false;
     for (Request* r : work) {
         r->next_pass++;
-        if (r->next_pass == (int)r->passes.size()) {
-            const PassBuf& last = r->passes.back();
-            sums.push_back(SummaryItem{last.flags, (int)last.cells, r->d_counts});
-        }
+        finished |= r->next_pass == (int)r->passes.size();
     }
-    if (e == cudaSuccess && !sums.empty()) e = launch_summary_items(sums.data(), (int)sums.size(), stream, &nl);
     // downloads of the requests that finished in this step, on the download stream after the step
-    if (e == cudaSuccess && !sums.empty()) {
+    if (e == cudaSuccess && finished) {
         cudaEvent_t computed = nullptr;
         e = cudaEventCreateWithFlags(&computed, cudaEventDisableTiming);
         if (e == cudaSuccess) {

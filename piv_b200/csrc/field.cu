@@ -82,14 +82,8 @@ struct PlaceBatch {
 
 struct ValidateBatch {
     int n;
-    int cell_start[kMaxBatch + 1];
+    int tile_start[kMaxBatch + 1];
     ValidateParams item[kMaxBatch];
-};
-
-struct SummaryBatch {
-    int n;
-    int cell_start[kMaxBatch + 1];
-    SummaryItem item[kMaxBatch];
 };
 
 __global__ void place_kernel(const __grid_constant__ PlaceBatch b) {
@@ -100,6 +94,8 @@ __global__ void place_kernel(const __grid_constant__ PlaceBatch b) {
     const int k = u - b.cell_start[it];
     const int ix = k % p.grid.nx, iy = k / p.grid.nx;
     const int n = p.grid.window;
+    if (k == 0 && p.zero_counts)
+        for (int j = 0; j < 5; ++j) p.zero_counts[j] = 0;
     // max = (w - n).saturating_sub(1) (multipass.rs:207-208)
     const float max_x = (float)max(p.W - n - 1, 0), max_y = (float)max(p.H - n - 1, 0);
     float2 shift = make_float2(0.0f, 0.0f);
@@ -238,123 +234,167 @@ __device__ __forceinline__ float residual8(float value, const int (&k)[8], int c
     return __fdiv_rn(fabsf(__fsub_rn(value, med)), __fadd_rn(median8(dev, c), eps));
 }
 
-__device__ int collect_neighbours(const float* dx, const float* dy, const uint8_t* snap, int nx, int ny, int ix, int iy,
-                                  int radius, float* nu, float* nv) {
+// Usable neighbours within `radius` of (x, y) of a tile stored with row stride `stride`: flags in f
+// (cells outside the field are not usable there), values in u, v; appended to nu, nv.
+template <int RU, int RF>
+__device__ int collect_neighbours(const float (*u)[RU], const float (*v)[RU], const uint8_t (*f)[RF], int vy, int vx,
+                                  int fy, int fx, int radius, float* nu, float* nv) {
     int c = 0;
-    const int y0 = max(iy - radius, 0), y1 = min(iy + radius, ny - 1);
-    const int x0 = max(ix - radius, 0), x1 = min(ix + radius, nx - 1);
-    for (int y = y0; y <= y1; ++y)
-        for (int x = x0; x <= x1; ++x)
-            if (!(x == ix && y == iy) && (snap[y * nx + x] & F_INVALID) == 0) {
-                nu[c] = dx[y * nx + x];
-                nv[c] = dy[y * nx + x];
+    for (int j = -radius; j <= radius; ++j)
+        for (int i = -radius; i <= radius; ++i)
+            if ((i || j) && (f[fy + j][fx + i] & F_INVALID) == 0) {
+                nu[c] = u[vy + j][vx + i];
+                nv[c] = v[vy + j][vx + i];
                 ++c;
             }
     return c;
 }
 
-// Per-vector tests (validate.rs:59-78).
-__device__ __forceinline__ void validate_vector(const ValidateParams& p, int k) {
-    uint8_t f = p.flags0[k];
-    if (!(f & F_NO_SIGNAL)) {
-        if (hypotf(p.dx[k], p.dy[k]) > p.max_displacement) f |= F_OUT_OF_RANGE;
-        if (p.ppr[k] < p.ppr_threshold) f |= F_LOW_PPR;
-    }
-    p.flags1[k] = f;
-}
+// Validation of one 32 x TY tile of a field in one launch: the per-vector tests (validate.rs:59-78)
+// on the tile and a halo of 3 cells, the normalized median test (:80-100) on the tile and a halo of
+// 2, the replacement by the median of usable neighbours at radius 1, then 2 (:102-128) on the tile,
+// and on the last pass the summary counts (:40-46). The flag snapshots between the stages stay in
+// shared memory; the halo cells are computed again by each tile that needs them (TY = 32: 1.27
+// times the median tests of separate launches; TY = 8: 1.69 times).
+//
+// The stages are short and their launches were not: as three kernels with flag planes in memory and
+// two more for the summary, each pass of a small field spent 13 us in them and the last one 6 us
+// more (31 x 31 cells, B200); a 512 x 512 pair of one pass went from 48.6 to 39.1 us and a
+// batch of 64 pairs of 1280 x 800 from 4.17 to 3.76 ms with this and the export below.
+constexpr int kTileX = 32;
+constexpr int kValidateThreads = 256;
 
-// Normalized median test on a snapshot of the flags (validate.rs:80-100).
-__device__ __forceinline__ void validate_median(const ValidateParams& p, int k) {
-    const int ix = k % p.nx, iy = k / p.nx;
-    uint8_t f = p.flags1[k];
-    if ((f & F_INVALID) == 0) {
-        // usable 3x3 neighbours (validate.rs:133-155), padded slots for the others
-        int ku[8], kv[8];
-        int c = 0;
+template <int TY>
+__global__ void __launch_bounds__(kValidateThreads) validate_kernel(const __grid_constant__ ValidateBatch b) {
+    constexpr int LX = kTileX + 6, LY = TY + 6;  // values and first flags
+    constexpr int MX = kTileX + 4, MY = TY + 4;  // flags after the median test
+    __shared__ float su[LY][LX], sv[LY][LX];
+    __shared__ uint8_t s1[LY][LX], s2[MY][MX];
+    __shared__ unsigned int s_count[5];
+    const int it = batch_item(b.tile_start, b.n, (int)blockIdx.x);
+    const ValidateParams& p = b.item[it];
+    const int tile = (int)blockIdx.x - b.tile_start[it], tiles_x = (p.nx + kTileX - 1) / kTileX;
+    const int x0 = (tile % tiles_x) * kTileX, y0 = (tile / tiles_x) * TY;
+    if (threadIdx.x < 5) s_count[threadIdx.x] = 0;
+    for (int i = threadIdx.x; i < LX * LY; i += kValidateThreads) {
+        const int ly = i / LX, lx = i - ly * LX, x = x0 + lx - 3, y = y0 + ly - 3;
+        uint8_t f = F_NO_SIGNAL;  // outside the field: not usable
+        float u = 0.0f, v = 0.0f;
+        if (x >= 0 && x < p.nx && y >= 0 && y < p.ny) {
+            const int k = y * p.nx + x;
+            f = p.flags0[k];
+            u = p.dx[k];
+            v = p.dy[k];
+            if (!(f & F_NO_SIGNAL)) {
+                if (hypotf(u, v) > p.max_displacement) f |= F_OUT_OF_RANGE;
+                if (p.ppr[k] < p.ppr_threshold) f |= F_LOW_PPR;
+            }
+        }
+        su[ly][lx] = u;
+        sv[ly][lx] = v;
+        s1[ly][lx] = f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < MX * MY; i += kValidateThreads) {
+        const int my = i / MX, mx = i - my * MX, ly = my + 1, lx = mx + 1;
+        uint8_t f = s1[ly][lx];
+        if ((f & F_INVALID) == 0) {
+            // usable 3x3 neighbours (validate.rs:133-155), padded slots for the others
+            int ku[8], kv[8];
+            int c = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int dxo = (j < 3) ? j - 1 : (j < 5 ? (j == 3 ? -1 : 1) : j - 6);
-            const int dyo = (j < 3) ? -1 : (j < 5 ? 0 : 1);
-            const int x = ix + dxo, y = iy + dyo;
-            ku[j] = kv[j] = 0x7fffffff;
-            if (x >= 0 && x < p.nx && y >= 0 && y < p.ny) {
-                const int o = y * p.nx + x;
-                if ((p.flags1[o] & F_INVALID) == 0) {
-                    ku[j] = tkey(p.dx[o]);
-                    kv[j] = tkey(p.dy[o]);
-                    ++c;
+            for (int j = 0; j < 8; ++j) {
+                const int dxo = (j < 3) ? j - 1 : (j < 5 ? (j == 3 ? -1 : 1) : j - 6);
+                const int dyo = (j < 3) ? -1 : (j < 5 ? 0 : 1);
+                const bool use = (s1[ly + dyo][lx + dxo] & F_INVALID) == 0;
+                ku[j] = use ? tkey(su[ly + dyo][lx + dxo]) : 0x7fffffff;
+                kv[j] = use ? tkey(sv[ly + dyo][lx + dxo]) : 0x7fffffff;
+                c += use;
+            }
+            if (c >= 2) {
+                sort8(ku);
+                sort8(kv);
+                const float ru = residual8(su[ly][lx], ku, c, p.median_eps);
+                const float rv = residual8(sv[ly][lx], kv, c, p.median_eps);
+                if (__fsqrt_rn(__fadd_rn(__fmul_rn(ru, ru), __fmul_rn(rv, rv))) > p.median_threshold) f |= F_MEDIAN_OUTLIER;
+            }
+        }
+        s2[my][mx] = f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kTileX * TY; i += kValidateThreads) {
+        const int ty = i / kTileX, tx = i % kTileX, x = x0 + tx, y = y0 + ty;
+        const bool in = x < p.nx && y < p.ny;
+        uint8_t f = 0;
+        if (in) {
+            f = s2[ty + 2][tx + 2];
+            float u = su[ty + 3][tx + 3], v = sv[ty + 3][tx + 3];
+            if (p.replace && (f & F_NO_SIGNAL) == 0 && (f & F_INVALID) != 0) {
+                float nu[24], nv[24];
+                bool done = false;
+                for (int radius = 1; radius <= 2 && !done; ++radius) {
+                    const int c = collect_neighbours<LX, MX>(su, sv, s2, ty + 3, tx + 3, ty + 2, tx + 2, radius, nu, nv);
+                    if (c > 0) {
+                        u = median_sorted(nu, c);
+                        v = median_sorted(nv, c);
+                        f |= F_REPLACED;
+                        done = true;
+                    }
+                }
+                if (!done) {
+                    u = NAN;
+                    v = NAN;
                 }
             }
+            const int k = y * p.nx + x;
+            p.out_dx[k] = u;
+            p.out_dy[k] = v;
+            p.out_flags[k] = f;
         }
-        if (c >= 2) {
-            sort8(ku);
-            sort8(kv);
-            const float ru = residual8(p.dx[k], ku, c, p.median_eps);
-            const float rv = residual8(p.dy[k], kv, c, p.median_eps);
-            if (__fsqrt_rn(__fadd_rn(__fmul_rn(ru, ru), __fmul_rn(rv, rv))) > p.median_threshold) f |= F_MEDIAN_OUTLIER;
-        }
-    }
-    p.flags2[k] = f;
-}
-
-// Replacement by the median of usable neighbours at radius 1, then 2 (validate.rs:102-128).
-__device__ __forceinline__ void validate_replace(const ValidateParams& p, int k) {
-    const int ix = k % p.nx, iy = k / p.nx;
-    uint8_t f = p.flags2[k];
-    float u = p.dx[k], v = p.dy[k];
-    if (p.replace && (f & F_NO_SIGNAL) == 0 && (f & F_INVALID) != 0) {
-        float nu[24], nv[24];
-        bool done = false;
-        for (int radius = 1; radius <= 2 && !done; ++radius) {
-            const int c = collect_neighbours(p.dx, p.dy, p.flags2, p.nx, p.ny, ix, iy, radius, nu, nv);
-            if (c > 0) {
-                u = median_sorted(nu, c);
-                v = median_sorted(nv, c);
-                f |= F_REPLACED;
-                done = true;
+        if (p.counts) {  // the same branch for the whole block; every lane takes part in the ballots
+            const bool none = f & F_NO_SIGNAL;
+            const bool bit[5] = {none, !none && (f & F_LOW_PPR), !none && (f & F_MEDIAN_OUTLIER),
+                                 !none && (f & F_OUT_OF_RANGE), !none && (f & F_REPLACED)};
+#pragma unroll
+            for (int j = 0; j < 5; ++j) {
+                const unsigned m = __ballot_sync(0xffffffffu, in && bit[j]);
+                if (m && (threadIdx.x & 31) == 0) atomicAdd(&s_count[j], (unsigned)__popc(m));
             }
         }
-        if (!done) {
-            u = NAN;
-            v = NAN;
-        }
     }
-    p.out_dx[k] = u;
-    p.out_dy[k] = v;
-    p.out_flags[k] = f;
+    if (!p.counts) return;
+    __syncthreads();
+    if (threadIdx.x < 5 && s_count[threadIdx.x])
+        atomicAdd(&p.counts[threadIdx.x], (unsigned long long)s_count[threadIdx.x]);
 }
 
-template <int STAGE>
-__global__ void validate_kernel(const __grid_constant__ ValidateBatch b) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= b.cell_start[b.n]) return;
-    const int it = batch_item(b.cell_start, b.n, u);
-    const int k = u - b.cell_start[it];
-    if (STAGE == 0) validate_vector(b.item[it], k);
-    if (STAGE == 1) validate_median(b.item[it], k);
-    if (STAGE == 2) validate_replace(b.item[it], k);
-}
+// Tile height: 32 rows when the batch then still has two tiles per SM, else 8 (a field of 31 x 31
+// cells is 4 tiles of 8 rows; 1000 x 1000 cells are 1024 tiles of 32).
+constexpr long long kTallTileCells = 148ll * 2 * kTileX * 32;
 
 cudaError_t launch_validate_items(const ValidateParams* items, int count, cudaStream_t s, int* launches) {
     for (int off = 0; off < count; off += kMaxBatch) {
         ValidateBatch b;
         b.n = min(count - off, kMaxBatch);
+        long long cells = 0;
+        for (int i = 0; i < b.n; ++i) cells += (long long)items[off + i].nx * items[off + i].ny;
+        const int ty = cells >= kTallTileCells ? 32 : 8;
         long long total = 0;
         for (int i = 0; i < b.n; ++i) {
             b.item[i] = items[off + i];
-            b.cell_start[i] = (int)total;
-            total += (long long)b.item[i].nx * b.item[i].ny;
+            b.tile_start[i] = (int)total;
+            total += (long long)((b.item[i].nx + kTileX - 1) / kTileX) * ((b.item[i].ny + ty - 1) / ty);
         }
-        b.cell_start[b.n] = (int)total;
+        b.tile_start[b.n] = (int)total;
         if (total <= 0) continue;
         if (total > 0x7fffffffll) return cudaErrorInvalidValue;
-        const unsigned blocks = (unsigned)((total + 255) / 256);
-        validate_kernel<0><<<blocks, 256, 0, s>>>(b);
-        validate_kernel<1><<<blocks, 256, 0, s>>>(b);
-        validate_kernel<2><<<blocks, 256, 0, s>>>(b);
+        if (ty == 32)
+            validate_kernel<32><<<(unsigned)total, kValidateThreads, 0, s>>>(b);
+        else
+            validate_kernel<8><<<(unsigned)total, kValidateThreads, 0, s>>>(b);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        if (launches) *launches += 3;
+        if (launches) ++*launches;
     }
     return cudaSuccess;
 }
@@ -362,62 +402,61 @@ cudaError_t launch_validate_items(const ValidateParams* items, int count, cudaSt
 cudaError_t launch_validate(const ValidateParams& p, cudaStream_t s) { return launch_validate_items(&p, 1, s, nullptr); }
 
 // ---------------------------------------------------------------------------------------------
-// Summary counts (validate.rs:40-46), from the final flags as `validate` counts them.
+// Final fields to the caller's device buffers: one launch for all arrays of all items (a copy
+// command each had cost a batch of 64 pairs 256 of them, about 1.5 us apiece).
 // ---------------------------------------------------------------------------------------------
-__global__ void summary_zero_kernel(const __grid_constant__ SummaryBatch b) {
-    const int i = threadIdx.x / 5, j = threadIdx.x % 5;
-    if (i < b.n) b.item[i].counts5[j] = 0;
-}
+struct ExportBatch {
+    int n;
+    int block_start[kMaxBatch + 1];
+    ExportItem item[kMaxBatch];
+};
+constexpr int kExportThreads = 256, kExportCells = 4 * kExportThreads;
 
-__global__ void summary_kernel(const __grid_constant__ SummaryBatch b) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = u < b.cell_start[b.n];
-    const int it = in ? batch_item(b.cell_start, b.n, u) : 0;
-    unsigned int loc[5] = {0, 0, 0, 0, 0};
-    if (in) {
-        const uint8_t f = b.item[it].flags[u - b.cell_start[it]];
-        if (f & F_NO_SIGNAL) {
-            loc[0] = 1;
-        } else {
-            loc[1] = (f & F_LOW_PPR) ? 1 : 0;
-            loc[2] = (f & F_MEDIAN_OUTLIER) ? 1 : 0;
-            loc[3] = (f & F_OUT_OF_RANGE) ? 1 : 0;
-            loc[4] = (f & F_REPLACED) ? 1 : 0;
-        }
-    }
-    // Lanes of one item reduce together; the leader of each item's lanes adds the totals.
-    const unsigned same = __match_any_sync(0xffffffffu, in ? it : -1);
-    const int leader = __ffs(same) - 1;
+__global__ void __launch_bounds__(kExportThreads) export_kernel(const __grid_constant__ ExportBatch b) {
+    const int it = batch_item(b.block_start, b.n, (int)blockIdx.x);
+    const ExportItem& q = b.item[it];
+    const int base = ((int)blockIdx.x - b.block_start[it]) * kExportCells;
+    if (base == 0 && threadIdx.x < 5 && q.out_counts) q.out_counts[threadIdx.x] = q.counts[threadIdx.x];
+    const float* const src[3] = {q.dx, q.dy, q.ppr};
+    float* const dst[3] = {q.out_dx, q.out_dy, q.out_ppr};
+    const uintptr_t at = (uintptr_t)q.dx | (uintptr_t)q.dy | (uintptr_t)q.ppr | (uintptr_t)q.out_dx | (uintptr_t)q.out_dy |
+                         (uintptr_t)q.out_ppr;
+    const uintptr_t at1 = (uintptr_t)q.flags | (uintptr_t)q.out_flags;
+    if (at % 16 == 0 && at1 % 4 == 0 && base + kExportCells <= q.n) {
+        const int k = base + 4 * threadIdx.x;
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
-        const unsigned int v = __reduce_add_sync(same, loc[i]);
-        if (in && (int)(threadIdx.x & 31) == leader && v) atomicAdd(&b.item[it].counts5[i], (unsigned long long)v);
+        for (int j = 0; j < 3; ++j)
+            if (dst[j]) *reinterpret_cast<float4*>(dst[j] + k) = *reinterpret_cast<const float4*>(src[j] + k);
+        if (q.out_flags) *reinterpret_cast<uchar4*>(q.out_flags + k) = *reinterpret_cast<const uchar4*>(q.flags + k);
+        return;
+    }
+    for (int k = base + threadIdx.x; k < min(base + kExportCells, q.n); k += kExportThreads) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            if (dst[j]) dst[j][k] = src[j][k];
+        if (q.out_flags) q.out_flags[k] = q.flags[k];
     }
 }
 
-cudaError_t launch_summary_items(const SummaryItem* items, int count, cudaStream_t s, int* launches) {
+cudaError_t launch_export_items(const ExportItem* items, int count, cudaStream_t s, int* launches) {
     for (int off = 0; off < count; off += kMaxBatch) {
-        SummaryBatch b;
+        ExportBatch b;
         b.n = min(count - off, kMaxBatch);
         long long total = 0;
         for (int i = 0; i < b.n; ++i) {
             b.item[i] = items[off + i];
-            b.cell_start[i] = (int)total;
-            total += b.item[i].n;
+            b.block_start[i] = (int)total;
+            total += ((long long)b.item[i].n + kExportCells - 1) / kExportCells;
         }
-        b.cell_start[b.n] = (int)total;
-        summary_zero_kernel<<<1, 5 * kMaxBatch, 0, s>>>(b);
-        if (total > 0) summary_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(b);
+        b.block_start[b.n] = (int)total;
+        if (total <= 0) continue;
+        if (total > 0x7fffffffll) return cudaErrorInvalidValue;
+        export_kernel<<<(unsigned)total, kExportThreads, 0, s>>>(b);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        if (launches) *launches += total > 0 ? 2 : 1;
+        if (launches) ++*launches;
     }
     return cudaSuccess;
-}
-
-cudaError_t launch_summary(const uint8_t* flags, int n, unsigned long long* counts5, cudaStream_t s) {
-    SummaryItem it{flags, n, counts5};
-    return launch_summary_items(&it, 1, s, nullptr);
 }
 
 }  // namespace pivb200

@@ -108,6 +108,7 @@ struct PlaceParams {
     int use_stats;
     StatsView sa, sb;
     float min_mean, min_std;
+    unsigned long long* zero_counts;  // nullable: 5 summary counters set to 0 (the pair's first pass)
 };
 
 cudaError_t launch_place(const PlaceParams& p, cudaStream_t s);
@@ -121,29 +122,35 @@ struct ValidateParams {
     const float* dy;
     const float* ppr;
     const uint8_t* flags0;  // raw flags (0 / NO_SIGNAL)
-    uint8_t* flags1;        // scratch: after per-vector tests
-    uint8_t* flags2;        // scratch: after the median test
     float* out_dx;
     float* out_dy;
     uint8_t* out_flags;
     float max_displacement, ppr_threshold, median_threshold, median_eps;
     int replace;
+    // nullable: adds the summary counts of the validated flags (validate.rs:40-46: no_signal,
+    // low_ppr, median_outliers, out_of_range, replaced)
+    unsigned long long* counts;
 };
 
 cudaError_t launch_validate(const ValidateParams& p, cudaStream_t s);
 cudaError_t launch_validate_items(const ValidateParams* items, int count, cudaStream_t s, int* launches);
-constexpr int kValidateLaunches = 3;
+constexpr int kValidateLaunches = 1;
 
-// Summary counts from a validated flag field (validate.rs:40-46): no_signal, low_ppr,
-// median_outliers, out_of_range, replaced.
-cudaError_t launch_summary(const uint8_t* flags, int n, unsigned long long* counts5, cudaStream_t s);
-constexpr int kSummaryLaunches = 2;
-struct SummaryItem {
+// A validated field and where the caller wants it (device memory; null outputs are skipped).
+struct ExportItem {
+    const float* dx;
+    const float* dy;
+    const float* ppr;
     const uint8_t* flags;
+    const unsigned long long* counts;  // 5
     int n;
-    unsigned long long* counts5;
+    float* out_dx;
+    float* out_dy;
+    float* out_ppr;
+    uint8_t* out_flags;
+    unsigned long long* out_counts;
 };
-cudaError_t launch_summary_items(const SummaryItem* items, int count, cudaStream_t s, int* launches);
+cudaError_t launch_export_items(const ExportItem* items, int count, cudaStream_t s, int* launches);
 
 // ----------------------------------------------------------------------------- post-processing
 // Flow statistics of one validated field (flowstats.rs:67-101 via flow.rs:20-36); blocking.

@@ -8,25 +8,14 @@
 // cudaMalloc fail even though the pool has room. Such callers own every buffer they pass in and
 // need the library to allocate nothing.
 //
-// The validation stages need two per-cell flag snapshots (validate.rs:81 and :103 take them).
-// Here they live in one file-scope device array of fixed size, kNoAllocMaxCells cells per
-// snapshot (2 x 2,097,152 bytes = 4 MiB). Every GPU that loads this library holds that array
-// until the process exits. Fields with more cells are rejected.
+// The validation kernel keeps its flag snapshots (validate.rs:81 and :103 take them) in shared
+// memory, tile by tile, so it needs no scratch in device memory. The entry point is defined for
+// fields of at most kNoAllocMaxCells cells; larger ones are rejected.
 //
-// Host code cannot use the array's name as a device address (it names a host-side stand-in),
-// so the address is taken with cudaGetSymbolAddress once per device, with that device current,
-// on the first call of the entry point on that device. Make that first call before any stream
-// capture begins. The address is kept for the life of the process, so the entry point must not
-// be used on a device after cudaDeviceReset (or any reset of its primary context). Every call
-// shares the same array, and the kernels overwrite every snapshot byte they later read, so
-// nothing needs clearing between calls; two calls whose work overlaps on the GPU (different
-// streams, or different host threads on one device) race on it.
-//
-// Outputs must not overlap inputs: the median test reads neighbours' dx/dy while other threads
-// write theirs, so in-place validation would race. Overlapping buffers are rejected.
+// Outputs must not overlap inputs: a tile reads its neighbours' dx/dy while other blocks write
+// theirs, so in-place validation would race. Overlapping buffers are rejected.
 #include <cstdint>
 #include <cstdio>
-#include <mutex>
 #include <string>
 
 #include "../../include/piv_b200.h"
@@ -37,29 +26,6 @@ using namespace pivb200;
 namespace {
 
 constexpr long long kNoAllocMaxCells = 1ll << 21;
-
-static __device__ __align__(256) uint8_t g_validate_scratch[2 * kNoAllocMaxCells];
-
-constexpr int kMaxDevices = 64;
-std::mutex g_mu;
-uint8_t* g_scratch_addr[kMaxDevices] = {};
-
-// Device address of the scratch array on the current device (taken once per device).
-cudaError_t scratch_for_current_device(uint8_t** out) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (!g_scratch_addr[dev]) {
-        void* p = nullptr;
-        e = cudaGetSymbolAddress(&p, g_validate_scratch);
-        if (e != cudaSuccess) return e;
-        g_scratch_addr[dev] = static_cast<uint8_t*>(p);
-    }
-    *out = g_scratch_addr[dev];
-    return cudaSuccess;
-}
 
 int reject(int code, const std::string& msg) {
     set_last_error(msg.c_str());
@@ -87,7 +53,7 @@ int32_t piv_validate_field_noalloc(int64_t ny, int64_t nx, const float* dx, cons
     if (nx > kNoAllocMaxCells / ny) {
         char buf[200];
         snprintf(buf, sizeof(buf),
-                 "piv_validate_field_noalloc: a %lld x %lld field exceeds the fixed scratch of %lld cells",
+                 "piv_validate_field_noalloc: a %lld x %lld field exceeds the limit of %lld cells",
                  (long long)ny, (long long)nx, kNoAllocMaxCells);
         return reject(PIV_ERR_UNSUPPORTED, buf);
     }
@@ -105,14 +71,9 @@ int32_t piv_validate_field_noalloc(int64_t ny, int64_t nx, const float* dx, cons
             if (overlap(outs[o], out_bytes[o], outs[q], out_bytes[q]))
                 return reject(PIV_ERR_ARGUMENT, "piv_validate_field_noalloc: output buffers overlap");
     }
-    uint8_t* scratch = nullptr;
-    cudaError_t e = scratch_for_current_device(&scratch);
-    if (e != cudaSuccess)
-        return reject(PIV_ERR_CUDA, std::string("piv_validate_field_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-    ValidateParams vp{(int)nx, (int)ny, dx, dy, peak_ratio, flags, scratch, scratch + kNoAllocMaxCells,
-                      out_dx, out_dy, out_flags, max_displacement, ppr_threshold, median_threshold, median_eps,
-                      replace};
-    e = launch_validate(vp, static_cast<cudaStream_t>(stream));
+    ValidateParams vp{(int)nx, (int)ny, dx, dy, peak_ratio, flags, out_dx, out_dy, out_flags,
+                      max_displacement, ppr_threshold, median_threshold, median_eps, replace, nullptr};
+    const cudaError_t e = launch_validate(vp, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return reject(PIV_ERR_CUDA, std::string("piv_validate_field_noalloc: ") + cudaGetErrorString(e));
     return PIV_OK;
 }
