@@ -26,7 +26,7 @@ UNITS = {
     "noalloc.cu": ["--fmad=false"],
     "post.cu": ["--fmad=false"],
 }
-HEADERS = ["common.cuh", "fft.cuh", "kernels.h", "window.cuh", "tc.cuh"]
+HEADERS = ["common.cuh", "fft.cuh", "kernels.h", "window.cuh", "packed.cuh", "tc.cuh"]
 
 
 def _nvcc():

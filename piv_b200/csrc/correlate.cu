@@ -7,9 +7,10 @@
 // Work decomposition (one thread group = N*T threads, one PAIR of windows per group):
 //   1. both windows of the pair are sampled (bilinear, the reference's f32 operation order, no
 //      FMA) straight into registers, each as one complex plane z = a + i*b (frame A's window in
-//      the real part, frame B's in the imaginary part); lane (x, t) holds column x at rows
-//      t + T*p (32 and 64 px: the block of rows P*rev(t) + p, sampled one new row at a time), so
-//      each load instruction reads contiguous image rows;
+//      the real part, frame B's in the imaginary part); lane (x, t) samples column x at the block of
+//      rows P*rev(t) + p, one new row at a time, so each load instruction reads contiguous image
+//      rows; where the column pass wants the rows t + T*p (24, 48, 96 and 128 px), the T lanes of a
+//      column then exchange rows through shared memory;
 //   2. mean removal and energies (one group reduction of 4 sums for both windows), 2-D FFT of
 //      both planes at once: columns in registers, transpose through shared memory, rows in
 //      registers;
@@ -35,18 +36,18 @@
 namespace pivb200 {
 
 // Compile-time shape of one correlation kernel: window N, lanes per line T, window pairs or
-// single windows, groups per CTA G, minimum resident CTAs per SM (register cap), sampler.
+// single windows, groups per CTA G, minimum resident CTAs per SM (register cap).
 // G and MINB only change the launch geometry, never the arithmetic; N, T and PAIR fix the FFT
 // decomposition and therefore the rounding of the results.
-template <int N_, int T_, bool PAIR_, int G_, int MINB_, bool SHFL_ = false, bool DEFORM_ = false>
+template <int N_, int T_, bool PAIR_, int G_, int MINB_, bool DEFORM_ = false>
 struct CorrCfg {
     static constexpr int N = N_, T = T_, G = G_, MINB = MINB_;
-    static constexpr bool PAIR = PAIR_, SHFL_SAMPLE = SHFL_, DEFORM = DEFORM_;
-    // 32 and 64 px window pairs (uniform and deformed) sample in the block layout (lane t holds
-    // rows P*rev(t) + p) and run the column pass of the forward FFT from it (bit-reversed blocks
-    // in, lane t ends with the frequency rows t + T*k); every other configuration samples
-    // interleaved rows (t + T*p).
-    static constexpr bool BLOCK = PAIR && (N_ == 32 || N_ == 64);
+    static constexpr bool PAIR = PAIR_, DEFORM = DEFORM_;
+    // 32 and 64 px windows (and one-lane lines, where the layouts are the same) run the column pass
+    // of the forward FFT from the block layout (lane t holds rows P*rev(t) + p; bit-reversed blocks
+    // in, lane t ends with the frequency rows t + T*k), the others from interleaved rows (t + T*p).
+    // The two round differently, so a size keeps its own.
+    static constexpr bool BLOCK = T_ == 1 || N_ == 32 || N_ == 64;
     static constexpr int P = N / T;
     static constexpr int NT = N * T;
     static constexpr int THREADS = G * NT;
@@ -76,6 +77,12 @@ struct CorrCfg {
     __host__ __device__ static constexpr int AF(int row, int col) {
         return (BLOCK && T == 2) ? row * N + ((col + 2 * (((row >> 1) & 3) + 4 * (row & 1))) & (N - 1)) : A(row, col);
     }
+    // The exchange of sampled rows (stored as rows P*rev(t) + p, read as rows t + T*p, by the lanes of
+    // 16/T columns per half-warp): A on four lanes; on two (24 px), rows of 32 rotated by 8 where the
+    // row's parity and half differ, again 16 distinct bank pairs either way.
+    __host__ __device__ static constexpr int AX(int row, int col) {
+        return T == 2 ? row * 32 + ((col + 8 * ((row & 1) ^ (row >= P ? 1 : 0))) & 31) : A(row, col);
+    }
     __host__ __device__ static constexpr int B(int ky, int kx) {
         return T == 1 ? ky * LD + kx : ky * LD + (ky / P) * Q + kx + kx / P;
     }
@@ -96,7 +103,7 @@ struct CorrCfg {
     __host__ __device__ static constexpr int YO(int r, int x) { return r * N + (x ^ (((r & 1) << 3) | (r & 6))); }
     __host__ __device__ static constexpr int CP(int y, int x) { return y * N + x + 4 * (y >> 4); }
     static constexpr int CP_OFF = 2 * (N / 2 + 1) * N;
-    static_assert(!(BLOCK && T == 2) || N * N <= PLANE_ELEMS, "first-transpose plane");
+    static_assert(T != 2 || (N <= 32 && N * 32 <= PLANE_ELEMS), "planes of 32 per row");
     static_assert(PAIR || (N == 128 && BS(N - 1, N - 1) < PLANE_ELEMS &&
                            CP_OFF + CP(N - 1, N - 1) < 2 * PLANE_ELEMS &&
                            sizeof(float) * (size_t)(CP(N - 1, N - 1) + 1) <= PLANE1),
@@ -239,9 +246,8 @@ __device__ __forceinline__ unsigned eligible_rows(int by, int ex, int cx, int rt
 // Separates Z and its Hermitian partner M = Z[-k] into the cross spectrum (times 4):
 //   2FA = Z + conj(M), 2FB = -i (Z - conj(M)), C = conj(2FA) * 2FB.
 __device__ __forceinline__ float2 cross4(float2 z, float2 m) {
-    const float far = z.x + m.x, fai = z.y - m.y;
-    const float fbr = z.y + m.y, fbi = m.x - z.x;
-    return make_float2(far * fbr + fai * fbi, far * fbi - fai * fbr);
+    const float2 s = cadd(z, m), d = csub(z, m);  // s = (2FA.re, 2FB.re), d = (-2FB.im, 2FA.im)
+    return make_float2(__fmaf_rn(s.x, s.y, -__fmul_rn(d.x, d.y)), -__fmaf_rn(s.x, d.x, __fmul_rn(s.y, d.y)));
 }
 
 // One CTA's work: G window pairs (or single windows) of one item, `block` counting the item's
@@ -284,6 +290,7 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
         if constexpr (!C::DEFORM) org[wi] = active ? prm.origins[cell] : make_float4(0.f, 0.f, 0.f, 0.f);
         ok[wi] = active && prm.status[cell] != 0;
     }
+    const SeparateProduct mul(prm.ncells);
     if constexpr (C::DEFORM) {
 #pragma unroll
         for (int wi = 0; wi < WPG; ++wi) {
@@ -298,64 +305,66 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
             org[wi] = make_float4(corner_blend(k0.x, k0.z, k1.x, k1.z, 0.5f, 0.5f),
                                   corner_blend(k0.y, k0.w, k1.y, k1.w, 0.5f, 0.5f), 0.f, 0.f);
             if (wi == 0) {
-                sample_deformed<N, T, C::BLOCK>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, line,
-                                                C::BLOCK ? rt : t, s_ramp, z0);
+                sample_deformed<N>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, line, C::BLOCK ? P * rt : t,
+                                   C::BLOCK ? 1 : T, s_ramp, mul, z0);
             } else if constexpr (PAIR) {
-                sample_deformed<N, T, C::BLOCK>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, line,
-                                                C::BLOCK ? rt : t, s_ramp, z1);
+                sample_deformed<N>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, line, C::BLOCK ? P * rt : t,
+                                   C::BLOCK ? 1 : T, s_ramp, mul, z1);
             }
         }
-    } else if constexpr (C::BLOCK) {
-        const GlobalSrc ga{prm.img_a, prm.W}, gb{prm.img_b, prm.W};
-        sample_block<N, T, false, C::SHFL_SAMPLE>(ga, prm.H, prm.W, org[0].x, org[0].y, line, rt, z0);
-        sample_block<N, T, true, C::SHFL_SAMPLE>(gb, prm.H, prm.W, org[0].z, org[0].w, line, rt, z0);
-        sample_block<N, T, false, C::SHFL_SAMPLE>(ga, prm.H, prm.W, org[1].x, org[1].y, line, rt, z1);
-        sample_block<N, T, true, C::SHFL_SAMPLE>(gb, prm.H, prm.W, org[1].z, org[1].w, line, rt, z1);
-    } else if constexpr (C::SHFL_SAMPLE) {
-        const GlobalSrc ga{prm.img_a, prm.W}, gb{prm.img_b, prm.W};
-        sample_column<N, T, false>(ga, prm.H, prm.W, org[0].x, org[0].y, line, t, z0);
-        sample_column<N, T, true>(gb, prm.H, prm.W, org[0].z, org[0].w, line, t, z0);
-        if constexpr (PAIR) {
-            sample_column<N, T, false>(ga, prm.H, prm.W, org[1].x, org[1].y, line, t, z1);
-            sample_column<N, T, true>(gb, prm.H, prm.W, org[1].z, org[1].w, line, t, z1);
-        }
     } else {
-        const GlobalSrc ga{prm.img_a, prm.W}, gb{prm.img_b, prm.W};
-        sample_column_direct<N, T, false>(ga, prm.H, prm.W, org[0].x, org[0].y, line, t, z0);
-        sample_column_direct<N, T, true>(gb, prm.H, prm.W, org[0].z, org[0].w, line, t, z0);
-        if constexpr (PAIR) {
-            sample_column_direct<N, T, false>(ga, prm.H, prm.W, org[1].x, org[1].y, line, t, z1);
-            sample_column_direct<N, T, true>(gb, prm.H, prm.W, org[1].z, org[1].w, line, t, z1);
+        const PairSource p0 = pair_source(prm.img_a, prm.img_b, prm.H, prm.W, org[0], line);
+        const PairSource p1 = pair_source(prm.img_a, prm.img_b, prm.H, prm.W, org[WPG - 1], line);
+        if constexpr (C::BLOCK) {
+            if (p0.copy_a && p0.copy_b) copy_rows(p0, prm.W, P * rt, 1, z0); else stream_rows<N>(p0, prm.W, P * rt, mul, z0);
+            if constexpr (PAIR) {
+                if (p1.copy_a && p1.copy_b) copy_rows(p1, prm.W, P * rt, 1, z1); else stream_rows<N>(p1, prm.W, P * rt, mul, z1);
+            }
+        } else if (p0.copy_a && p0.copy_b && p1.copy_a && p1.copy_b) {  // the same for the whole group
+            copy_rows(p0, prm.W, t, T, z0);
+            if constexpr (PAIR) copy_rows(p1, prm.W, t, T, z1);
+        } else {
+            // streamed block rows, then the T lanes of a column exchange them for rows t + T*p; the planes
+            // are not written again before the group barriers of the sums below
+            const unsigned line_lanes = ((1u << T) - 1u) << ((threadIdx.x & 31) - t);
+            stream_rows<N>(p0, prm.W, P * rt, mul, z0);
+            if constexpr (PAIR) stream_rows<N>(p1, prm.W, P * rt, mul, z1);
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                plane0[C::AX(P * rt + p, line)] = z0[p];
+                if constexpr (PAIR) reinterpret_cast<float2*>(plane1_raw)[C::AX(P * rt + p, line)] = z1[p];
+            }
+            __syncwarp(line_lanes);
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                z0[p] = plane0[C::AX(t + T * p, line)];
+                if constexpr (PAIR) z1[p] = reinterpret_cast<float2*>(plane1_raw)[C::AX(t + T * p, line)];
+            }
+            __syncwarp(line_lanes);
         }
     }
     {
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 s0 = make_float2(0.f, 0.f), s1 = s0;
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            s.x += z0[p].x;
-            s.y += z0[p].y;
-            if constexpr (PAIR) {
-                s.z += z1[p].x;
-                s.w += z1[p].y;
-            }
+            s0 = cadd(s0, z0[p]);
+            if constexpr (PAIR) s1 = cadd(s1, z1[p]);
         }
-        s = group_sum4<C>(s, s_red, g, gt);
+        const float4 s = group_sum4<C>(make_float4(s0.x, s0.y, s1.x, s1.y), s_red, g, gt);
         constexpr float inv = 1.0f / (float)(N * N);
-        const float m0a = s.x * inv, m0b = s.y * inv, m1a = s.z * inv, m1b = s.w * inv;
-        float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float2 m0 = make_float2(__fmul_rn(s.x, inv), __fmul_rn(s.y, inv));
+        const float2 m1 = make_float2(__fmul_rn(s.z, inv), __fmul_rn(s.w, inv));
+        float2 e0 = make_float2(0.f, 0.f), e1 = e0;
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            z0[p].x = __fsub_rn(z0[p].x, m0a);
-            z0[p].y = __fsub_rn(z0[p].y, m0b);
-            e.x += z0[p].x * z0[p].x;
-            e.y += z0[p].y * z0[p].y;
+            z0[p] = csub(z0[p], m0);
+            e0 = cfma2(z0[p], z0[p], e0);
             if constexpr (PAIR) {
-                z1[p].x = __fsub_rn(z1[p].x, m1a);
-                z1[p].y = __fsub_rn(z1[p].y, m1b);
-                e.z += z1[p].x * z1[p].x;
-                e.w += z1[p].y * z1[p].y;
+                z1[p] = csub(z1[p], m1);
+                e1 = cfma2(z1[p], z1[p], e1);
             }
         }
+        float4 e = make_float4(e0.x, e0.y, e1.x, e1.y);
         e = group_sum4<C>(e, s_red, g, gt);
         // correlate.rs:110 (flat window) and :136 (scale 1 / (n^2 sqrt(Ea Eb))); the factor 1/4
         // undoes the 2x folded into each separated spectrum (exact power-of-two scaling).
@@ -378,12 +387,8 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
             plane1[C::AF(t + T * k, line)] = z1[k];
         }
     } else {
-        if constexpr (PAIR && N == 64) {
-            fft_line_interleaved2<N, T, 1>(z0, z1, t, s_roots);  // both windows stage by stage
-        } else {
-            fft_line_interleaved<N, T, 1>(z0, t, s_roots);
-            if constexpr (PAIR) fft_line_interleaved<N, T, 1>(z1, t, s_roots);
-        }
+        fft_line_interleaved<N, T, 1>(z0, t, s_roots);
+        if constexpr (PAIR) fft_line_interleaved<N, T, 1>(z1, t, s_roots);
 #pragma unroll
         for (int k = 0; k < P; ++k) {
             plane0[C::A(k + P * rt, line)] = z0[k];
@@ -477,8 +482,7 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
         // part); scale as the reference does (c *= scale).
 #pragma unroll
         for (int k = 0; k < P2; ++k) {
-            y[k].x = y[k].x * scale[0];
-            y[k].y = y[k].y * scale[0];
+            y[k] = cmul2(y[k], make_float2(scale[0], scale[0]));
             cplane[C::CP(k + P2 * rt2, x1)] = y[k].x;
             cplane[C::CP(k + P2 * rt2, x2)] = y[k].y;
         }
@@ -496,7 +500,7 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
         }
         group_argmax<C>(best.x, bi0, s_red, g, gt);
         if (!(best.x > -INFINITY)) bi0 = 0;
-        group_sync<C>(g);  // the scaled plane is complete in shared memory
+        group_sync<C>(g);  // the plane is complete in shared memory
         // Footprint of the primary peak (correlate.rs:242-254): half-width along +-y, +-x.
         if (gt < 4) {
             const int by = bi0 / N, bx = bi0 % N;
@@ -608,8 +612,7 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
         // Lane now holds corr[y = k + P*rt][x = line]; scale as the reference does (c *= scale).
 #pragma unroll
         for (int k = 0; k < P; ++k) {
-            z0[k].x = z0[k].x * scale[0];
-            z0[k].y = z0[k].y * scale[WPG - 1];
+            z0[k] = cmul2(z0[k], make_float2(scale[0], scale[WPG - 1]));
             plane0[C::A(k + P * rt, line)] = z0[k];
         }
 
@@ -634,7 +637,7 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
         group_argmax<C>(best.y, bi1, s_red, g, gt);
         if (!(best.x > -INFINITY)) bi0 = 0;
         if (!(best.y > -INFINITY)) bi1 = 0;
-        group_sync<C>(g);  // the scaled planes are complete in shared memory
+        group_sync<C>(g);  // the planes are complete in shared memory
         auto at = [&](int ch, int y, int x) -> float {
             const float2 v = plane0[C::A(y % N, x % N)];
             return ch == 0 ? v.x : v.y;
@@ -768,14 +771,14 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) correlate_kernel(const __
 // the FFT decomposition (N, T, PAIR) of that size's per-size kernel, so the results are bit
 // for bit those of the per-size launches.
 // ---------------------------------------------------------------------------------------------
-using FusedC0 = CorrCfg<8, 1, true, 32, 2, true>;
-using FusedC1 = CorrCfg<16, 1, true, 16, 2, false>;
-using FusedC2 = CorrCfg<32, 2, true, 4, 2, false>;
-using FusedC3 = CorrCfg<64, 4, true, 1, 2, false>;
-using FusedC4 = CorrCfg<8, 1, true, 32, 2, false, true>;
-using FusedC5 = CorrCfg<16, 1, true, 16, 2, false, true>;
-using FusedC6 = CorrCfg<32, 2, true, 4, 2, false, true>;
-using FusedC7 = CorrCfg<64, 4, true, 1, 2, false, true>;
+using FusedC0 = CorrCfg<8, 1, true, 32, 2>;
+using FusedC1 = CorrCfg<16, 1, true, 16, 2>;
+using FusedC2 = CorrCfg<32, 2, true, 4, 2>;
+using FusedC3 = CorrCfg<64, 4, true, 1, 2>;
+using FusedC4 = CorrCfg<8, 1, true, 32, 2, true>;
+using FusedC5 = CorrCfg<16, 1, true, 16, 2, true>;
+using FusedC6 = CorrCfg<32, 2, true, 4, 2, true>;
+using FusedC7 = CorrCfg<64, 4, true, 1, 2, true>;
 constexpr int kFusedThreads = 256;
 constexpr size_t kFusedSmem =
     std::max({FusedC0::SMEM, FusedC1::SMEM, FusedC2::SMEM, FusedC3::SMEM, FusedC4::SMEM, FusedC5::SMEM, FusedC6::SMEM,
@@ -890,36 +893,28 @@ bool corr_supported(int n) {
 
 // ---------------------------------------------------------------------------------------------
 // Launch variants per window size. Within one size every variant has the same N, T and PAIR,
-// so all of them compute bit-identical results; they differ in groups per CTA, register cap and
-// sampler. Variant 0 is the default; the autotuner (api.cu) times the others on live data.
+// so all of them compute bit-identical results; they differ in groups per CTA and register cap.
+// Variant 0 is the default; the autotuner (api.cu) times the others on live data.
 // ---------------------------------------------------------------------------------------------
 struct CorrVariant {
     const char* name;
     cudaError_t (*launch)(CorrBatch, cudaStream_t);
 };
 
-#define PIV_V(N, T, PR, G, MB, SH) {#N "/T" #T "/G" #G "/B" #MB "/" #SH, &launch_t<CorrCfg<N, T, PR, G, MB, SH>>}
-static const CorrVariant kV8[] = {PIV_V(8, 1, true, 32, 1, false), PIV_V(8, 1, true, 16, 2, false),
-                                  PIV_V(8, 1, true, 32, 2, true), PIV_V(8, 1, true, 4, 16, false)};
-static const CorrVariant kV12[] = {PIV_V(12, 1, true, 16, 1, false), PIV_V(12, 1, true, 8, 3, false),
-                                   PIV_V(12, 1, true, 16, 2, true)};
-static const CorrVariant kV16[] = {PIV_V(16, 1, true, 16, 2, false), PIV_V(16, 1, true, 8, 4, false),
-                                   PIV_V(16, 1, true, 8, 3, false), PIV_V(16, 1, true, 16, 2, true),
-                                   PIV_V(16, 1, true, 8, 4, true), PIV_V(16, 1, true, 2, 16, false),
-                                   PIV_V(16, 1, true, 4, 8, false), PIV_V(16, 1, true, 2, 16, true)};
-static const CorrVariant kV24[] = {PIV_V(24, 2, true, 4, 2, true), PIV_V(24, 2, true, 4, 2, false),
-                                   PIV_V(24, 2, true, 2, 4, true)};
-static const CorrVariant kV32[] = {PIV_V(32, 2, true, 4, 2, false), PIV_V(32, 2, true, 4, 2, true),
-                                   PIV_V(32, 2, true, 2, 4, true), PIV_V(32, 2, true, 2, 3, true),
-                                   PIV_V(32, 2, true, 1, 8, true), PIV_V(32, 2, true, 1, 8, false)};
-static const CorrVariant kV48[] = {PIV_V(48, 4, true, 1, 2, true), PIV_V(48, 4, true, 1, 2, false),
-                                   PIV_V(48, 4, true, 1, 1, true)};
-static const CorrVariant kV64[] = {PIV_V(64, 4, true, 1, 2, false), PIV_V(64, 4, true, 1, 2, true),
-                                   PIV_V(64, 4, true, 1, 1, true)};
-static const CorrVariant kV96[] = {PIV_V(96, 4, true, 1, 1, true), PIV_V(96, 4, true, 1, 1, false)};
-static const CorrVariant kV128[] = {PIV_V(128, 4, false, 1, 1, false), PIV_V(128, 4, false, 1, 1, true)};
+#define PIV_V(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB, &launch_t<CorrCfg<N, T, PR, G, MB>>}
+static const CorrVariant kV8[] = {PIV_V(8, 1, true, 32, 3), PIV_V(8, 1, true, 16, 2), PIV_V(8, 1, true, 4, 16)};
+static const CorrVariant kV12[] = {PIV_V(12, 1, true, 16, 1), PIV_V(12, 1, true, 8, 3)};
+static const CorrVariant kV16[] = {PIV_V(16, 1, true, 16, 2), PIV_V(16, 1, true, 8, 4), PIV_V(16, 1, true, 8, 3),
+                                   PIV_V(16, 1, true, 2, 16), PIV_V(16, 1, true, 4, 8)};
+static const CorrVariant kV24[] = {PIV_V(24, 2, true, 4, 2), PIV_V(24, 2, true, 2, 4)};
+static const CorrVariant kV32[] = {PIV_V(32, 2, true, 4, 2), PIV_V(32, 2, true, 2, 4), PIV_V(32, 2, true, 2, 3),
+                                   PIV_V(32, 2, true, 1, 8)};
+static const CorrVariant kV48[] = {PIV_V(48, 4, true, 1, 2), PIV_V(48, 4, true, 1, 1)};
+static const CorrVariant kV64[] = {PIV_V(64, 4, true, 1, 2), PIV_V(64, 4, true, 1, 1)};
+static const CorrVariant kV96[] = {PIV_V(96, 4, true, 1, 1)};
+static const CorrVariant kV128[] = {PIV_V(128, 4, false, 1, 1)};
 // Deformed-window variants: the same FFT decomposition per size, the deformed sampler.
-#define PIV_D(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB "/deform", &launch_t<CorrCfg<N, T, PR, G, MB, false, true>>}
+#define PIV_D(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB "/deform", &launch_t<CorrCfg<N, T, PR, G, MB, true>>}
 static const CorrVariant kD8[] = {PIV_D(8, 1, true, 32, 1)};
 static const CorrVariant kD12[] = {PIV_D(12, 1, true, 16, 1)};
 static const CorrVariant kD16[] = {PIV_D(16, 1, true, 16, 2), PIV_D(16, 1, true, 8, 4)};

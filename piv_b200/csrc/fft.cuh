@@ -12,8 +12,8 @@
 //      twiddle w_N^(p*t), P-point DFT in registers.
 //      Lane t ends with X[t + T*k1] (interleaved).
 //
-// The first is used for the forward transforms and for the last inverse stage, the second for
-// the first inverse stage, so the data never has to be re-ordered inside a lane.
+// The second is used for the forward column pass and the first inverse stage, the first for the
+// forward row pass and the last inverse stage, so the data never has to be re-ordered inside a lane.
 //
 // Unnormalized DFT, forward kernel exp(-2 pi i j k / N), inverse exp(+2 pi i j k / N) — the
 // definition rustfft/realfft implement (the reference's FFT crates, rust/Cargo.lock:1644-1646,
@@ -21,6 +21,8 @@
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include "packed.cuh"
 
 namespace pivb200 {
 
@@ -46,9 +48,6 @@ template <int N>
 __device__ __forceinline__ float2 croot(int k) {
     return c_roots[root_off(N) + k];
 }
-
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 
 // a * w (DIR = +1) or a * conj(w) (DIR = -1); w is a forward root.
 template <int DIR>
@@ -92,18 +91,19 @@ __device__ __forceinline__ void butterfly(float2 (&t)[R]) {
         float2 a0 = cadd(t[0], t[2]), a1 = csub(t[0], t[2]);
         float2 b0 = cadd(t[1], t[3]), b1 = mul_mi<DIR>(csub(t[1], t[3]));
         t[0] = cadd(a0, b0);
-        t[1] = cadd(a1, b1);
         t[2] = csub(a0, b0);
-        t[3] = csub(a1, b1);
+        // b1 is a swapped pair: its sums stay scalar, so that no moves are spent on pairing it
+        t[1] = make_float2(a1.x + b1.x, a1.y + b1.y);
+        t[3] = make_float2(a1.x - b1.x, a1.y - b1.y);
     } else {
         static_assert(R == 3, "radix");
         constexpr float kS3 = 0.866025403784438646763723f;  // sqrt(3)/2
         float2 s = cadd(t[1], t[2]), d = csub(t[1], t[2]);
-        float2 m = make_float2(t[0].x - 0.5f * s.x, t[0].y - 0.5f * s.y);
+        float2 m = cfma2(s, make_float2(-0.5f, -0.5f), t[0]);
         float2 r = mul_mi<DIR>(make_float2(kS3 * d.x, kS3 * d.y));
         t[0] = cadd(t[0], s);
-        t[1] = cadd(m, r);
-        t[2] = csub(m, r);
+        t[1] = make_float2(m.x + r.x, m.y + r.y);
+        t[2] = make_float2(m.x - r.x, m.y - r.y);
     }
 }
 
@@ -146,6 +146,15 @@ __device__ __forceinline__ void dft_reg(float2 (&x)[P]) {
     for (int i = 0; i < P; ++i) x[i] = y[i];
 }
 
+// s * a + o, the signed add of the cross-lane stages (s = +1 or -1). Packed, except at 64 points,
+// where the pairs it forms make the kernel spill more (64 px pass of a 2048 x 2048 pair 504 us packed,
+// 495 scalar; 96 px 688 packed, 706 scalar; 128 px 543 and 557).
+template <int N>
+__device__ __forceinline__ float2 signed_add(float s, float2 a, float2 o) {
+    if constexpr (N == 64) return make_float2(fmaf(s, a.x, o.x), fmaf(s, a.y, o.y));
+    return cfma2(make_float2(s, s), a, o);
+}
+
 template <int T>
 __device__ __forceinline__ int bitrev(int t) {
     int r = 0;
@@ -177,7 +186,7 @@ __device__ __forceinline__ void xlane_dif(float2 (&x)[P], int t, const float2* s
                 float2 o;
                 o.x = __shfl_xor_sync(0xffffffffu, x[i].x, h);
                 o.y = __shfl_xor_sync(0xffffffffu, x[i].y, h);
-                const float2 v = make_float2(fmaf(sg, x[i].x, o.x), fmaf(sg, x[i].y, o.y));
+                const float2 v = signed_add<N>(sg, x[i], o);
                 x[i] = quarter ? mul_mi<DIR>(v) : v;
             }
         } else {
@@ -187,7 +196,7 @@ __device__ __forceinline__ void xlane_dif(float2 (&x)[P], int t, const float2* s
                 float2 o;
                 o.x = __shfl_xor_sync(0xffffffffu, x[i].x, h);
                 o.y = __shfl_xor_sync(0xffffffffu, x[i].y, h);
-                x[i] = cmulw<DIR>(make_float2(fmaf(sg, x[i].x, o.x), fmaf(sg, x[i].y, o.y)), w);
+                x[i] = cmulw<DIR>(signed_add<N>(sg, x[i], o), w);
             }
         }
     }
@@ -220,7 +229,7 @@ __device__ __forceinline__ void xlane_dit(float2 (&x)[P], int t, const float2* s
                 float2 o;
                 o.x = __shfl_xor_sync(0xffffffffu, v.x, h);
                 o.y = __shfl_xor_sync(0xffffffffu, v.y, h);
-                x[i] = make_float2(fmaf(sg, v.x, o.x), fmaf(sg, v.y, o.y));
+                x[i] = signed_add<N>(sg, v, o);
             }
         } else {
             const float2 w = s_roots[(t & (h - 1)) * (N / (2 * h))];
@@ -262,9 +271,8 @@ __device__ __forceinline__ void fft_line_blocked(float2 (&x)[N / T], int t, cons
 
 // Two lines at once (the two windows of a pair), stage by stage: the same operations per value as
 // two calls of fft_line_interleaved (so the same results), ordered so that one line's shuffles
-// overlap the other's arithmetic. Measured per window size, it is used where it is faster: 64
-// points on four lanes (2.37 -> 2.20 ms for the c5 64 px pass; 32 points on two lanes 2.00 ->
-// 2.05, 96 points 2.247 -> 2.256).
+// overlap the other's arithmetic. Used at 32 and 64 points (2.37 -> 2.20 ms for the 64 px pass of a
+// 4096 x 4096 pair at 75 % overlap); at 24, 48 and 96 points the order makes no difference (0.3 %).
 template <int N, int T, int DIR>
 __device__ __forceinline__ void fft_line_interleaved2(float2 (&x)[N / T], float2 (&y)[N / T], int t,
                                                       const float2* s_roots) {
@@ -291,8 +299,8 @@ __device__ __forceinline__ void fft_line_interleaved2(float2 (&x)[N / T], float2
                     o.y = __shfl_xor_sync(0xffffffffu, x[i].y, h);
                     q.x = __shfl_xor_sync(0xffffffffu, y[i].x, h);
                     q.y = __shfl_xor_sync(0xffffffffu, y[i].y, h);
-                    const float2 v = make_float2(fmaf(sg, x[i].x, o.x), fmaf(sg, x[i].y, o.y));
-                    const float2 u = make_float2(fmaf(sg, y[i].x, q.x), fmaf(sg, y[i].y, q.y));
+                    const float2 v = signed_add<N>(sg, x[i], o);
+                    const float2 u = signed_add<N>(sg, y[i], q);
                     x[i] = quarter ? mul_mi<DIR>(v) : v;
                     y[i] = quarter ? mul_mi<DIR>(u) : u;
                 }
@@ -305,8 +313,8 @@ __device__ __forceinline__ void fft_line_interleaved2(float2 (&x)[N / T], float2
                     o.y = __shfl_xor_sync(0xffffffffu, x[i].y, h);
                     q.x = __shfl_xor_sync(0xffffffffu, y[i].x, h);
                     q.y = __shfl_xor_sync(0xffffffffu, y[i].y, h);
-                    x[i] = cmulw<DIR>(make_float2(fmaf(sg, x[i].x, o.x), fmaf(sg, x[i].y, o.y)), w);
-                    y[i] = cmulw<DIR>(make_float2(fmaf(sg, y[i].x, q.x), fmaf(sg, y[i].y, q.y)), w);
+                    x[i] = cmulw<DIR>(signed_add<N>(sg, x[i], o), w);
+                    y[i] = cmulw<DIR>(signed_add<N>(sg, y[i], q), w);
                 }
             }
         }
@@ -342,8 +350,8 @@ __device__ __forceinline__ void fft_line_blocked2(float2 (&x)[N / T], float2 (&y
                     o.y = __shfl_xor_sync(0xffffffffu, v.y, h);
                     q.x = __shfl_xor_sync(0xffffffffu, u.x, h);
                     q.y = __shfl_xor_sync(0xffffffffu, u.y, h);
-                    x[i] = make_float2(fmaf(sg, v.x, o.x), fmaf(sg, v.y, o.y));
-                    y[i] = make_float2(fmaf(sg, u.x, q.x), fmaf(sg, u.y, q.y));
+                    x[i] = signed_add<N>(sg, v, o);
+                    y[i] = signed_add<N>(sg, u, q);
                 }
             } else {
                 const float2 w = s_roots[(t & (h - 1)) * (N / (2 * h))];
