@@ -71,6 +71,91 @@ GridP to_gp(const PivGridC& g) {
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// Device blocks of destroyed frames and of the blocking stage calls, kept for the next ones: a
+// program that makes frames for every pair spent more time in cudaMalloc and cudaFree than in the
+// analysis (1024 x 768 pair, host to host: 1.55 ms and more, 0.32 ms with the blocks kept). A block comes here only when no work can be using it (its giver has waited for the device or for its
+// stream). At most kKeptBytes are kept per device, in no one's name; they go back to the device when
+// an allocation fails and when the device's last analyzer is destroyed.
+constexpr size_t kKeptBytes = (size_t)256 << 20;
+struct KeptBlocks {
+    std::multimap<size_t, void*> free;
+    size_t bytes = 0;
+    int analyzers = 0;  // live analyzers on the device
+};
+std::mutex g_kept_mu;
+std::map<int, KeptBlocks> g_kept;
+
+void drop_kept(KeptBlocks& k) {  // with g_kept_mu held and the device current
+    for (auto& b : k.free) cudaFree(b.second);
+    k.free.clear();
+    k.bytes = 0;
+}
+
+// cudaMalloc on the current device that first gives the kept blocks back when memory runs out.
+cudaError_t device_malloc(void** out, size_t bytes) {
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lk(g_kept_mu);
+        auto it = g_kept.find(dev);
+        if (it == g_kept.end() || it->second.free.empty()) return e;
+        drop_kept(it->second);
+    }
+    cudaGetLastError();  // not a sticky error
+    return cudaMalloc(out, bytes);
+}
+
+size_t block_bytes(size_t bytes) { return (bytes + 0xffff) & ~(size_t)0xffff; }  // multiples of 64 KiB
+
+// A block of at least `bytes` on the current device; give it back with the same `bytes`.
+template <class T>
+cudaError_t take_block(T** out, size_t bytes) {
+    const size_t want = block_bytes(bytes);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lk(g_kept_mu);
+        KeptBlocks& k = g_kept[dev];
+        auto it = k.free.find(want);
+        if (it != k.free.end()) {
+            *out = static_cast<T*>(it->second);
+            k.free.erase(it);
+            k.bytes -= want;
+            return cudaSuccess;
+        }
+    }
+    void* p = nullptr;
+    e = device_malloc(&p, want);
+    *out = static_cast<T*>(p);
+    return e;
+}
+
+// Hands a block of device `dev` (current) that nothing uses any more to the next taker.
+void give_block(int dev, void* p, size_t bytes) {
+    if (!p) return;
+    const size_t size = block_bytes(bytes);
+    {
+        std::lock_guard<std::mutex> lk(g_kept_mu);
+        KeptBlocks& k = g_kept[dev];
+        if (k.analyzers > 0 && k.bytes + size <= kKeptBytes) {
+            k.free.emplace(size, p);
+            k.bytes += size;
+            return;
+        }
+    }
+    cudaFree(p);
+}
+
+void count_analyzer(int dev, int by) {
+    std::lock_guard<std::mutex> lk(g_kept_mu);
+    KeptBlocks& k = g_kept[dev];
+    k.analyzers += by;
+    if (k.analyzers == 0) drop_kept(k);
+}
+
 struct PassBuf {
     PivGridC grid;
     int64_t cells;
@@ -135,6 +220,7 @@ struct PivAnalyzer {
     cudaGraphExec_t gexec = nullptr;
     std::vector<uintptr_t> gkey, pending_key;
     long long gnl = 0;  // kernels in the graph
+    bool counted = false;  // made by piv_analyzer_create
 
     bool mask_trivial() const { return min_mean <= 0.0f && min_std <= 0.0f; }
     std::vector<int32_t> pass_windows() const {
@@ -163,6 +249,14 @@ struct PivFrame {
     size_t d_raw_bytes = 0;
     float* d_bg = nullptr;
 };
+
+namespace {
+constexpr int kFrameWords = 4 + 512 + 4;
+// One block holds the image, the scratch words and the two scales.
+size_t frame_block_bytes(const PivFrame* f) {
+    return align256(sizeof(float) * (size_t)f->H * (size_t)f->W) + align256(sizeof(unsigned int) * (kFrameWords + 2));
+}
+}  // namespace
 
 struct PivBatch {
     PivAnalyzer* an = nullptr;  // private analyzer: its workspace is never resized by other calls
@@ -248,7 +342,7 @@ int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
         proto.push_back(pb);
     }
     const size_t total = align256(sizeof(unsigned long long) * 8 * (size_t)K) + per_pair * (size_t)K;
-    CUDA_TRY(cudaMalloc(&an->arena, total));
+    CUDA_TRY(device_malloc(&an->arena, total));
     char* p = (char*)an->arena;
     auto take = [&](size_t bytes) {
         void* r = p;
@@ -286,8 +380,8 @@ bool needs_stats(const PivAnalyzer* an, const PivFrame* f) { return !an->mask_tr
 int alloc_stats(PivFrame* f) {
     if (f->sum) return PIV_OK;
     const size_t cells = (size_t)(f->H + 1) * (size_t)(f->W + 1);
-    CUDA_TRY(cudaMalloc(&f->sum, sizeof(long long) * cells));
-    CUDA_TRY(cudaMalloc(&f->sumsq, sizeof(long long) * cells));
+    CUDA_TRY(take_block(&f->sum, sizeof(long long) * cells));
+    CUDA_TRY(take_block(&f->sumsq, sizeof(long long) * cells));
     return PIV_OK;
 }
 
@@ -534,8 +628,8 @@ int prepare_common(PivAnalyzer* an, PivFrame* f, const void* raw_dev, int32_t dt
     const bool chain = pre->smooth_sigma > 0.0f || pre->normalize_radius > 0;
     f->nonneg = dtype != PIV_DTYPE_F32 || bg_dev != nullptr;
     const size_t n = (size_t)f->H * (size_t)f->W;
-    if (chain && !f->base_store) CUDA_TRY(cudaMalloc(&f->base_store, sizeof(float) * n));
-    if (pre->smooth_sigma > 0.0f && pre->normalize_radius > 0 && !f->tmp) CUDA_TRY(cudaMalloc(&f->tmp, sizeof(float) * n));
+    if (chain && !f->base_store) CUDA_TRY(take_block(&f->base_store, sizeof(float) * n));
+    if (pre->smooth_sigma > 0.0f && pre->normalize_radius > 0 && !f->tmp) CUDA_TRY(take_block(&f->tmp, sizeof(float) * n));
     f->base = chain ? f->base_store : f->image;
     const bool stats = needs_stats(an, f);
     if (stats) {
@@ -572,10 +666,13 @@ int prepare_common(PivAnalyzer* an, PivFrame* f, const void* raw_dev, int32_t dt
 
 int stage_raw(PivFrame* f, size_t bytes) {
     if (f->d_raw_bytes >= bytes) return PIV_OK;
-    if (f->d_raw) CUDA_TRY(cudaFree(f->d_raw));
+    if (f->d_raw) {
+        CUDA_TRY(cudaDeviceSynchronize());
+        give_block(f->device, f->d_raw, f->d_raw_bytes);
+    }
     f->d_raw = nullptr;
     f->d_raw_bytes = 0;
-    CUDA_TRY(cudaMalloc(&f->d_raw, bytes));
+    CUDA_TRY(take_block(&f->d_raw, bytes));
     f->d_raw_bytes = bytes;
     return PIV_OK;
 }
@@ -647,6 +744,8 @@ int32_t piv_analyzer_create(const PivConfigC* cfg, PivAnalyzer** out) {
         return fail(PIV_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
     }
     an->cur = an->own;
+    an->counted = true;
+    count_analyzer(dev, 1);
     *out = an;
     return PIV_OK;
 }
@@ -668,6 +767,7 @@ void piv_analyzer_destroy(PivAnalyzer* an) {
     }
     if (an->arena) cudaFree(an->arena);
     if (an->own) cudaStreamDestroy(an->own);
+    if (an->counted) count_analyzer(an->device, -1);
     delete an;
 }
 
@@ -779,14 +879,13 @@ int32_t piv_frame_create(PivAnalyzer* an, int64_t height, int64_t width, PivFram
     f->device = an->device;
     f->H = height;
     f->W = width;
-    const size_t n = (size_t)height * (size_t)width;
-    cudaError_t e = cudaMalloc(&f->image, sizeof(float) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&f->words, sizeof(unsigned int) * (4 + 512 + 4));
-    if (e == cudaSuccess) e = cudaMalloc(&f->scales, sizeof(int) * 2);
+    const cudaError_t e = take_block(&f->image, frame_block_bytes(f));
     if (e != cudaSuccess) {
-        piv_frame_destroy(f);
+        delete f;
         return fail(PIV_ERR_CUDA, "frame allocation: %s", cudaGetErrorString(e));
     }
+    f->words = (unsigned int*)((char*)f->image + align256(sizeof(float) * (size_t)height * (size_t)width));
+    f->scales = (int*)(f->words + kFrameWords);
     f->base = f->image;
     *out = f;
     return PIV_OK;
@@ -794,17 +893,25 @@ int32_t piv_frame_create(PivAnalyzer* an, int64_t height, int64_t width, PivFram
 
 void piv_frame_destroy(PivFrame* f) {
     if (!f) return;
-    // A frame may outlive its analyzer: touch nothing of it. cudaFree synchronises the device.
+    // A frame may outlive its analyzer: touch nothing of it. Work that reads the frame may be queued on
+    // any stream, so its blocks are handed on only when the device is idle.
     cudaSetDevice(f->device);
-    cudaFree(f->image);
-    cudaFree(f->base_store);
-    cudaFree(f->tmp);
-    cudaFree(f->sum);
-    cudaFree(f->sumsq);
-    cudaFree(f->scales);
-    cudaFree(f->words);
-    cudaFree(f->d_raw);
-    cudaFree(f->d_bg);
+    if (cudaDeviceSynchronize() == cudaSuccess) {
+        const size_t n = sizeof(float) * (size_t)f->H * (size_t)f->W;
+        const size_t table = sizeof(long long) * (size_t)(f->H + 1) * (size_t)(f->W + 1);
+        give_block(f->device, f->image, frame_block_bytes(f));
+        give_block(f->device, f->base_store, n);
+        give_block(f->device, f->tmp, n);
+        give_block(f->device, f->sum, table);
+        give_block(f->device, f->sumsq, table);
+        give_block(f->device, f->d_raw, f->d_raw_bytes);
+        give_block(f->device, f->d_bg, n);
+    } else {  // a failed device, or a capture in progress: nothing of this frame is handed on
+        cudaGetLastError();
+        for (void* p : {(void*)f->image, (void*)f->base_store, (void*)f->tmp, (void*)f->sum, (void*)f->sumsq, f->d_raw,
+                        (void*)f->d_bg})
+            cudaFree(p);
+    }
     delete f;
 }
 
@@ -830,7 +937,7 @@ int32_t piv_frame_prepare(PivAnalyzer* an, PivFrame* f, const void* raw, int32_t
     CUDA_TRY(cudaMemcpyAsync(f->d_raw, raw, es * n, cudaMemcpyHostToDevice, an->cur));
     const float* bg = nullptr;
     if (background) {
-        if (!f->d_bg) CUDA_TRY(cudaMalloc(&f->d_bg, sizeof(float) * n));
+        if (!f->d_bg) CUDA_TRY(take_block(&f->d_bg, sizeof(float) * n));
         CUDA_TRY(cudaMemcpyAsync(f->d_bg, background, sizeof(float) * n, cudaMemcpyHostToDevice, an->cur));
         bg = f->d_bg;
     }
@@ -848,7 +955,7 @@ int32_t piv_frame_set_prepared(PivAnalyzer* an, PivFrame* f, const float* image,
     if (st) return st;
     const float* bsrc = f->image;
     if (base) {
-        if (!f->base_store) CUDA_TRY(cudaMalloc(&f->base_store, sizeof(float) * n));
+        if (!f->base_store) CUDA_TRY(take_block(&f->base_store, sizeof(float) * n));
         CUDA_TRY(cudaMemcpyAsync(f->base_store, base, sizeof(float) * n, cudaMemcpyHostToDevice, an->cur));
         bsrc = f->base_store;
     }
@@ -1042,7 +1149,8 @@ int place_windows(PivAnalyzer* an, int64_t height, int64_t width, const PivGridC
     const size_t c = (size_t)(grid->nx * grid->ny);
     const size_t pc = pred_grid ? (size_t)(pred_grid->nx * pred_grid->ny) : 0;
     void* buf = nullptr;
-    CUDA_TRY(cudaMalloc(&buf, align256(16 * c) + align256(c) + 2 * align256(4 * pc + 4) + align256(32 * c)));
+    const size_t buf_bytes = align256(16 * c) + align256(c) + 2 * align256(4 * pc + 4) + align256(32 * c);
+    CUDA_TRY(take_block(&buf, buf_bytes));
     char* p = (char*)buf;
     float4* d_org = (float4*)p;
     p += align256(16 * c);
@@ -1075,7 +1183,10 @@ int place_windows(PivAnalyzer* an, int64_t height, int64_t width, const PivGridC
     if (e == cudaSuccess) e = cudaMemcpyAsync(origins, d_org, 16 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && corners) e = cudaMemcpyAsync(corners, d_corners, 32 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess) e = cudaStreamSynchronize(an->cur);
-    cudaFree(buf);
+    if (e == cudaSuccess)
+        give_block(an->device, buf, buf_bytes);  // the stream has been waited for
+    else
+        cudaFree(buf);
     if (e != cudaSuccess) return fail(PIV_ERR_CUDA, "place: %s", cudaGetErrorString(e));
     return PIV_OK;
 }
@@ -1114,7 +1225,8 @@ int32_t piv_correlate_origins(PivAnalyzer* an, const PivFrame* a, const PivFrame
     if (use_stats && !(a->stats_valid && b->stats_valid)) return fail(PIV_ERR_ARGUMENT, "frame statistics missing");
     const size_t c = (size_t)ncells;
     void* buf = nullptr;
-    CUDA_TRY(cudaMalloc(&buf, align256(16 * c) + align256(c) + 3 * align256(4 * c) + align256(c) + 256));
+    const size_t buf_bytes = align256(16 * c) + align256(c) + 3 * align256(4 * c) + align256(c) + 256;
+    CUDA_TRY(take_block(&buf, buf_bytes));
     char* p = (char*)buf;
     float4* d_org = (float4*)p;
     p += align256(16 * c);
@@ -1152,7 +1264,10 @@ int32_t piv_correlate_origins(PivAnalyzer* an, const PivFrame* a, const PivFrame
     if (e == cudaSuccess && peak_ratio) e = cudaMemcpyAsync(peak_ratio, d_ppr, 4 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && flags) e = cudaMemcpyAsync(flags, d_fl, c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess) e = cudaStreamSynchronize(an->cur);
-    cudaFree(buf);
+    if (e == cudaSuccess)
+        give_block(an->device, buf, buf_bytes);  // the stream has been waited for
+    else
+        cudaFree(buf);
     if (e != cudaSuccess) return fail(PIV_ERR_CUDA, "correlate: %s", cudaGetErrorString(e));
     return check_device_error(an->device);
 }
@@ -1183,7 +1298,8 @@ int32_t piv_correlate_deform(PivAnalyzer* an, const PivFrame* a, const PivFrame*
     if (use_stats && !(a->stats_valid && b->stats_valid)) return fail(PIV_ERR_ARGUMENT, "frame statistics missing");
     const size_t c = (size_t)ncells;
     void* buf = nullptr;
-    CUDA_TRY(cudaMalloc(&buf, align256(16 * c) + align256(32 * c) + align256(c) + 3 * align256(4 * c) + align256(c) + 256));
+    const size_t buf_bytes = align256(16 * c) + align256(32 * c) + align256(c) + 3 * align256(4 * c) + align256(c) + 256;
+    CUDA_TRY(take_block(&buf, buf_bytes));
     char* p = (char*)buf;
     float4* d_org = (float4*)p;
     p += align256(16 * c);
@@ -1222,7 +1338,10 @@ int32_t piv_correlate_deform(PivAnalyzer* an, const PivFrame* a, const PivFrame*
     if (e == cudaSuccess && peak_ratio) e = cudaMemcpyAsync(peak_ratio, d_ppr, 4 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && flags) e = cudaMemcpyAsync(flags, d_fl, c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess) e = cudaStreamSynchronize(an->cur);
-    cudaFree(buf);
+    if (e == cudaSuccess)
+        give_block(an->device, buf, buf_bytes);  // the stream has been waited for
+    else
+        cudaFree(buf);
     if (e != cudaSuccess) return fail(PIV_ERR_CUDA, "correlate: %s", cudaGetErrorString(e));
     return PIV_OK;
 }
@@ -1321,7 +1440,8 @@ int32_t piv_validate_field(PivAnalyzer* an, int64_t ny, int64_t nx, const float*
     if (st) return st;
     const size_t c = (size_t)(ny * nx);
     void* buf = nullptr;
-    CUDA_TRY(cudaMalloc(&buf, 5 * align256(4 * c) + 2 * align256(c) + 256));
+    const size_t buf_bytes = 5 * align256(4 * c) + 2 * align256(c) + 256;
+    CUDA_TRY(take_block(&buf, buf_bytes));
     char* p = (char*)buf;
     auto take = [&](size_t bytes) {
         void* r = p;
@@ -1351,7 +1471,10 @@ int32_t piv_validate_field(PivAnalyzer* an, int64_t ny, int64_t nx, const float*
     if (e == cudaSuccess && out_flags) e = cudaMemcpyAsync(out_flags, fo, c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess) e = cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess) e = cudaStreamSynchronize(an->cur);
-    cudaFree(buf);
+    if (e == cudaSuccess)
+        give_block(an->device, buf, buf_bytes);  // the stream has been waited for
+    else
+        cudaFree(buf);
     if (e != cudaSuccess) return fail(PIV_ERR_CUDA, "validate: %s", cudaGetErrorString(e));
     if (summary) {
         summary->no_signal = (int64_t)hc[0];
@@ -1448,9 +1571,9 @@ int32_t piv_batch_create(const PivAnalyzer* parent, int64_t height, int64_t widt
     const size_t c = (size_t)bt->cells * (size_t)pairs;
     cudaError_t e = cudaStreamCreateWithFlags(&an->own, cudaStreamNonBlocking);
     an->cur = an->own;
-    if (e == cudaSuccess) e = cudaMalloc(&bt->raw, bt->frame_bytes * (size_t)nf);
+    if (e == cudaSuccess) e = device_malloc(&bt->raw, bt->frame_bytes * (size_t)nf);
     if (e == cudaSuccess)
-        e = cudaMalloc(&bt->out, align256(4 * c) * 3 + align256(c) + align256(8 * sizeof(unsigned long long) * pairs));
+        e = device_malloc(&bt->out, align256(4 * c) * 3 + align256(c) + align256(8 * sizeof(unsigned long long) * pairs));
     if (e != cudaSuccess) {
         piv_batch_destroy(bt);
         return fail(PIV_ERR_CUDA, "batch allocation: %s", cudaGetErrorString(e));
@@ -2010,7 +2133,7 @@ int admit_request(PivServer* sv, Request* r, bool inject_failure) {
             f->sum = (long long*)take(8 * (size_t)(r->H + 1) * (size_t)(r->W + 1));
             f->sumsq = (long long*)take(8 * (size_t)(r->H + 1) * (size_t)(r->W + 1));
         }
-        f->words = (unsigned int*)take(4 * (4 + 512 + 4));
+        f->words = (unsigned int*)take(4 * kFrameWords);
         f->scales = (int*)take(8);
     }
     for (PassBuf& pb : r->passes) {
