@@ -163,6 +163,53 @@ __device__ __forceinline__ void fix_stats(long long sum1, long long sum2, const 
     *std_out = dd_to_float(dd_sqrt(var));
 }
 
+// fix_stats without conversions, divisions or an IEEE square root, for scales that are plain powers of
+// two (fix_stats_fast_ok) and many pixels: the local normalisation is bound by instructions, and 64-bit
+// conversions and the reciprocals inside divisions run at an eighth of the FMA rate.
+//   - an int64 (below 2^62) is split into 23-bit pieces that become floats by their bit patterns;
+//   - a quotient by the small integer `count` is x * rc corrected by its exact remainder, and the root
+//     is x * rsqrt(x), refined once, corrected by its exact remainder (Karp and Markstein, "High
+//     precision division and square root", 1997): both accurate to about 2^-47, as fix_stats is, so the
+//     rounded results differ from its only within that distance of a rounding boundary.
+// rc is 1 / count rounded to nearest; p1, p2 are 2^-s1, 2^-s2.
+__device__ __forceinline__ bool fix_stats_fast_ok(const FixScale& fs) {
+    return fs.s1 >= 0 && fs.s1 <= 100 && fs.s2 >= 0 && fs.s2 <= 100;
+}
+
+__device__ __forceinline__ dfloat dd_from_bits(long long v, float scale) {
+    const float f2 = __fsub_rn(__int_as_float(0x4b400000 + (int)(v >> 46)), 12582912.0f);
+    const float f1 = __fsub_rn(__int_as_float(0x4b000000 | ((int)(v >> 23) & 0x7fffff)), 8388608.0f);
+    const float f0 = __fsub_rn(__int_as_float(0x4b000000 | ((int)v & 0x7fffff)), 8388608.0f);
+    const dfloat a = dd_quick(__fmul_rn(f2, 70368744177664.0f), __fmul_rn(f1, 8388608.0f));  // exact
+    const dfloat r = dd_quick(a.hi, __fadd_rn(a.lo, f0));
+    return {__fmul_rn(r.hi, scale), __fmul_rn(r.lo, scale)};
+}
+
+__device__ __forceinline__ dfloat dd_div_rc(dfloat x, float d, float rc) {
+    const float q = __fmul_rn(x.hi, rc);
+    const dfloat p = dd_two_prod(q, d);
+    return dd_quick(q, __fmul_rn(__fadd_rn(__fsub_rn(__fsub_rn(x.hi, p.hi), p.lo), x.lo), rc));
+}
+
+__device__ __forceinline__ void fix_stats_fast(long long sum1, long long sum2, float p1, float p2, float count, float rc,
+                                               float* mean_out, float* std_out) {
+    const dfloat mean = dd_div_rc(dd_from_bits(sum1, p1), count, rc);
+    const dfloat ex2 = dd_div_rc(dd_from_bits(sum2, p2), count, rc);
+    const dfloat var = dd_add(ex2, dd_neg(dd_mul(mean, mean)));
+    *mean_out = dd_to_float(mean);
+    if (!(var.hi > 0.0f)) {
+        *std_out = 0.0f;
+        return;
+    }
+    const float y = rsqrtf(var.hi);
+    float g = __fmul_rn(var.hi, y), h = __fmul_rn(0.5f, y);
+    const float e = __fmaf_rn(-g, h, 0.5f);
+    g = __fmaf_rn(g, e, g);
+    h = __fmaf_rn(h, e, h);
+    const dfloat p = dd_two_prod(g, g);
+    *std_out = __fmaf_rn(__fadd_rn(__fsub_rn(__fsub_rn(var.hi, p.hi), p.lo), var.lo), h, g);
+}
+
 // Rust f32::clamp (NaN passes through).
 __device__ __forceinline__ float rclamp(float x, float lo, float hi) {
     if (x < lo) return lo;
