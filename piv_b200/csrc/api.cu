@@ -664,6 +664,35 @@ int prepare_common(PivAnalyzer* an, PivFrame* f, const void* raw_dev, int32_t dt
     return PIV_OK;
 }
 
+// prepare_common for frames of one size and type: plain conversions (no clip, blur, normalisation or
+// mask tables) of all frames go in one launch.
+int prepare_frames(PivAnalyzer* an, PivFrame* const* frames, const void* const* raw_dev, int count, int32_t dtype,
+                   const PivPreprocessC* pre, const float* bg_dev) {
+    const bool plain = dtype != PIV_DTYPE_F32 && pre && !(pre->clip_percentile > 0.0) && !(pre->smooth_sigma > 0.0f) &&
+                       pre->normalize_radius <= 0 && an->mask_trivial();
+    if (!plain) {
+        for (int i = 0; i < count; ++i) {
+            const int st = prepare_common(an, frames[i], raw_dev[i], dtype, pre, bg_dev);
+            if (st) return st;
+        }
+        return PIV_OK;
+    }
+    std::vector<float*> images(count);
+    for (int i = 0; i < count; ++i) {
+        PivFrame* f = frames[i];
+        f->nonneg = true;
+        f->base = f->image;
+        f->stats_valid = false;
+        f->strips = true;
+        images[i] = f->image;
+    }
+    int nl = 0;
+    CUDA_TRY(launch_convert_frames(raw_dev, images.data(), count, (int)frames[0]->H, (int)frames[0]->W,
+                                   dtype == PIV_DTYPE_U8 ? RAW_U8 : RAW_U16, bg_dev, an->cur, &nl));
+    an->launches += nl;
+    return PIV_OK;
+}
+
 int stage_raw(PivFrame* f, size_t bytes) {
     if (f->d_raw_bytes >= bytes) return PIV_OK;
     if (f->d_raw) {
@@ -1500,11 +1529,10 @@ namespace {
 int batch_record(PivBatch* bt) {
     PivAnalyzer* an = bt->an;
     const int nf = (int)bt->frames.size();
-    for (int i = 0; i < nf; ++i) {
-        int st = prepare_common(an, bt->frames[i], (const char*)bt->raw + (size_t)i * bt->frame_bytes, bt->dtype, &bt->pre,
-                                bt->background);
-        if (st) return st;
-    }
+    std::vector<const void*> raw(nf);
+    for (int i = 0; i < nf; ++i) raw[i] = (const char*)bt->raw + (size_t)i * bt->frame_bytes;
+    const int ps = prepare_frames(an, bt->frames.data(), raw.data(), nf, bt->dtype, &bt->pre, bt->background);
+    if (ps) return ps;
     std::vector<const PivFrame*> fa(bt->K), fb(bt->K);
     for (int k = 0; k < bt->K; ++k) {
         fa[k] = bt->sequential ? bt->frames[k] : bt->frames[2 * k];
@@ -1760,8 +1788,9 @@ int32_t piv_pipeline_submit(PivPipeline* pl, const void* frame_a, const void* fr
     CUDA_TRY(cudaEventRecord(s.uploaded, pl->up));
     CUDA_TRY(cudaStreamWaitEvent(pl->prep, s.uploaded, 0));
     s.an->cur = pl->prep;
-    int st = prepare_common(s.an, s.fa, s.fa->d_raw, pl->dtype, &pl->pre, pl->background);
-    if (!st) st = prepare_common(s.an, s.fb, s.fb->d_raw, pl->dtype, &pl->pre, pl->background);
+    PivFrame* const frames[2] = {s.fa, s.fb};
+    const void* const raw[2] = {s.fa->d_raw, s.fb->d_raw};
+    int st = prepare_frames(s.an, frames, raw, 2, pl->dtype, &pl->pre, pl->background);
     s.an->cur = pl->comp;
     if (st) return st;
     CUDA_TRY(cudaEventRecord(s.prepared, pl->prep));
@@ -2160,9 +2189,9 @@ int admit_request(PivServer* sv, Request* r, bool inject_failure) {
     if (ue == cudaSuccess) ue = cudaStreamWaitEvent(sv->stream, uploaded, 0);
     cudaEventDestroy(uploaded);
     CUDA_TRY(ue);
-    int st = prepare_common(&r->cfg, &r->fa, r->fa.d_raw, r->dtype, &r->pre, nullptr);
-    if (!st) st = prepare_common(&r->cfg, &r->fb, r->fb.d_raw, r->dtype, &r->pre, nullptr);
-    return st;
+    PivFrame* const frames[2] = {&r->fa, &r->fb};
+    const void* const raw[2] = {r->fa.d_raw, r->fb.d_raw};
+    return prepare_frames(&r->cfg, frames, raw, 2, r->dtype, &r->pre, nullptr);
 }
 
 }  // namespace

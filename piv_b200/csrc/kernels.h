@@ -194,6 +194,10 @@ struct PrepParams {
     unsigned int* maxbits;    // 2 scratch words: max |base|, max |blurred|
 };
 
+// Integer frames of one size straight to f32 images (no clip, no mask tables, no chain), the same
+// background subtracted from each when it is not null.
+cudaError_t launch_convert_frames(const void* const* raw, float* const* out, int count, int H, int W, int raw_type,
+                                  const float* background, cudaStream_t s, int* launches);
 // Runs the whole PreparedFrame::new chain; returns the number of kernels launched in *launches.
 cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches);
 // The reference's f64 IntegralImage tables, already copied into `sum` / `sumsq` (8 bytes per
