@@ -68,6 +68,12 @@ struct CorrCfg {
     // plane0: float2 N x LD; plane1: float2 (PAIR) or float (single) N x LD.
     static constexpr size_t PLANE0 = sizeof(float2) * (size_t)PLANE_ELEMS;
     static constexpr size_t PLANE1 = ((PAIR ? sizeof(float2) : sizeof(float)) * (size_t)PLANE_ELEMS + 15) / 16 * 16;
+    // One-lane lines of fewer than 16 columns: a half-warp spans groups, and both access patterns (a row's
+    // N columns, and a column's rows at stride N + 1) continue from one group's banks into the next's
+    // when groups are N bank pairs (mod 16) apart. (Half of the 8 and 12 px kernels' shared-memory
+    // wavefronts were conflicts: 8 px pass of a 2048 x 2048 pair 95 -> 83 us, 12 px 113 -> 103.)
+    static constexpr size_t GROUP =
+        PLANE0 + PLANE1 + (T == 1 && N < 16 ? ((N + 32 - (PLANE0 + PLANE1) / 8 % 16) % 16) * 8 : 0);
     __host__ __device__ static constexpr int A(int row, int col) { return row * LD + (row / P) * Q + col; }
     // The first transpose (column spectra -> rows): A, except for the block layout on T = 2 lanes,
     // whose stores (rows t + 2k of eight columns per half-warp) would meet its loads' layout on
@@ -108,7 +114,7 @@ struct CorrCfg {
                            CP_OFF + CP(N - 1, N - 1) < 2 * PLANE_ELEMS &&
                            sizeof(float) * (size_t)(CP(N - 1, N - 1) + 1) <= PLANE1),
                   "single-window planes");
-    static constexpr size_t SMEM = (size_t)G * (PLANE0 + PLANE1) + sizeof(float2) * N + sizeof(float) * (size_t)G * NSEG * 4 +
+    static constexpr size_t SMEM = (size_t)G * GROUP + sizeof(float2) * N + sizeof(float) * (size_t)G * NSEG * 4 +
                                    (DEFORM ? sizeof(float) * N : 0) + 64;
 };
 
@@ -262,9 +268,9 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
     const int line = gt / T;
     const int t = gt - line * T;
     const int rt = bitrev<T>(t);
-    float2* plane0 = reinterpret_cast<float2*>(sbase + (size_t)g * (C::PLANE0 + C::PLANE1));
-    char* plane1_raw = sbase + (size_t)g * (C::PLANE0 + C::PLANE1) + C::PLANE0;
-    float2* s_roots = reinterpret_cast<float2*>(sbase + (size_t)G * (C::PLANE0 + C::PLANE1));
+    float2* plane0 = reinterpret_cast<float2*>(sbase + (size_t)g * C::GROUP);
+    char* plane1_raw = sbase + (size_t)g * C::GROUP + C::PLANE0;
+    float2* s_roots = reinterpret_cast<float2*>(sbase + (size_t)G * C::GROUP);
     float* s_red = reinterpret_cast<float*>(s_roots + N);
     float* s_ramp = s_red + G * C::NSEG * 4;  // c / (N - 1) for c < N (deformed windows only)
     __shared__ int s_hw[G][8];
@@ -894,7 +900,10 @@ bool corr_supported(int n) {
 // ---------------------------------------------------------------------------------------------
 // Launch variants per window size. Within one size every variant has the same N, T and PAIR,
 // so all of them compute bit-identical results; they differ in groups per CTA and register cap.
-// Variant 0 is the default; the autotuner (api.cu) times the others on live data.
+// Variant 0 is the default: the fastest of register caps and group counts measured on 2048 x 2048 pairs
+// (12 px 103 -> 89 us from 12 to 24 warps per SM, 24 px 485 -> 457 and 48 px 567 -> 545 from 12 to 18, at
+// some spills; 16, 32 and 64 px lose more to spills than more warps give; deformed 8 px 202 -> 138 us, 12 px
+// 236 -> 167 from one CTA per SM to three); the autotuner (api.cu) times the others on live data.
 // ---------------------------------------------------------------------------------------------
 struct CorrVariant {
     const char* name;
@@ -902,26 +911,24 @@ struct CorrVariant {
 };
 
 #define PIV_V(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB, &launch_t<CorrCfg<N, T, PR, G, MB>>}
-static const CorrVariant kV8[] = {PIV_V(8, 1, true, 32, 3), PIV_V(8, 1, true, 16, 2), PIV_V(8, 1, true, 4, 16)};
-static const CorrVariant kV12[] = {PIV_V(12, 1, true, 16, 1), PIV_V(12, 1, true, 8, 3)};
-static const CorrVariant kV16[] = {PIV_V(16, 1, true, 16, 2), PIV_V(16, 1, true, 8, 4), PIV_V(16, 1, true, 8, 3),
-                                   PIV_V(16, 1, true, 2, 16), PIV_V(16, 1, true, 4, 8)};
-static const CorrVariant kV24[] = {PIV_V(24, 2, true, 4, 2), PIV_V(24, 2, true, 2, 4)};
-static const CorrVariant kV32[] = {PIV_V(32, 2, true, 4, 2), PIV_V(32, 2, true, 2, 4), PIV_V(32, 2, true, 2, 3),
-                                   PIV_V(32, 2, true, 1, 8)};
-static const CorrVariant kV48[] = {PIV_V(48, 4, true, 1, 2), PIV_V(48, 4, true, 1, 1)};
+static const CorrVariant kV8[] = {PIV_V(8, 1, true, 16, 6), PIV_V(8, 1, true, 32, 3), PIV_V(8, 1, true, 32, 4)};
+static const CorrVariant kV12[] = {PIV_V(12, 1, true, 16, 4), PIV_V(12, 1, true, 16, 3), PIV_V(12, 1, true, 8, 6)};
+static const CorrVariant kV16[] = {PIV_V(16, 1, true, 16, 2), PIV_V(16, 1, true, 8, 4), PIV_V(16, 1, true, 8, 5)};
+static const CorrVariant kV24[] = {PIV_V(24, 2, true, 2, 6), PIV_V(24, 2, true, 4, 3), PIV_V(24, 2, true, 2, 4)};
+static const CorrVariant kV32[] = {PIV_V(32, 2, true, 4, 2), PIV_V(32, 2, true, 2, 4), PIV_V(32, 2, true, 1, 8)};
+static const CorrVariant kV48[] = {PIV_V(48, 4, true, 1, 3), PIV_V(48, 4, true, 1, 2)};
 static const CorrVariant kV64[] = {PIV_V(64, 4, true, 1, 2), PIV_V(64, 4, true, 1, 1)};
 static const CorrVariant kV96[] = {PIV_V(96, 4, true, 1, 1)};
 static const CorrVariant kV128[] = {PIV_V(128, 4, false, 1, 1)};
 // Deformed-window variants: the same FFT decomposition per size, the deformed sampler.
 #define PIV_D(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB "/deform", &launch_t<CorrCfg<N, T, PR, G, MB, true>>}
-static const CorrVariant kD8[] = {PIV_D(8, 1, true, 32, 1)};
-static const CorrVariant kD12[] = {PIV_D(12, 1, true, 16, 1)};
+static const CorrVariant kD8[] = {PIV_D(8, 1, true, 32, 3)};
+static const CorrVariant kD12[] = {PIV_D(12, 1, true, 16, 3)};
 static const CorrVariant kD16[] = {PIV_D(16, 1, true, 16, 2), PIV_D(16, 1, true, 8, 4)};
-static const CorrVariant kD24[] = {PIV_D(24, 2, true, 4, 2)};
+static const CorrVariant kD24[] = {PIV_D(24, 2, true, 2, 5)};
 static const CorrVariant kD32[] = {PIV_D(32, 2, true, 4, 2), PIV_D(32, 2, true, 2, 4)};
-static const CorrVariant kD48[] = {PIV_D(48, 4, true, 1, 2)};
-static const CorrVariant kD64[] = {PIV_D(64, 4, true, 1, 2), PIV_D(64, 4, true, 1, 1)};
+static const CorrVariant kD48[] = {PIV_D(48, 4, true, 1, 3)};
+static const CorrVariant kD64[] = {PIV_D(64, 4, true, 1, 2)};
 static const CorrVariant kD96[] = {PIV_D(96, 4, true, 1, 1)};
 static const CorrVariant kD128[] = {PIV_D(128, 4, false, 1, 1)};
 #undef PIV_D
