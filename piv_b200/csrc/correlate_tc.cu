@@ -109,32 +109,42 @@ __device__ __forceinline__ uint32_t mnmaj_chunk(int rows, int m, int k) {
 
 // Window sampling for the tensor-core tier (correlate.rs:182-202 semantics: integer copy when
 // both fractional parts are < 1e-4, bilinear otherwise), one lane per column streaming down the
-// rows. Each lane loads both taps of every row itself from one row pointer (the right-hand tap
-// is the next float, or the same one at the right image border), with no shuffles and no
-// conditional loads; the row below is carried to the next iteration. The bilinear weights are
-// applied as two linear interpolations with FMA (rounding differs from the reference's weight
-// sum by an ulp, far below the split-BF16 precision); zero fractions make it an exact copy.
-template <int N, bool IMAG>
-__device__ __forceinline__ void sample_rows(const float* __restrict__ img, int H, int W, float ox, float oy, int x,
-                                            float2 (&z)[N]) {
-    const float fx0 = floorf(ox), fy0 = floorf(oy);
-    const int x0 = min(max((int)fx0, 0), W - 1), y0 = min(max((int)fy0, 0), H - 1);
-    float tx = ox - fx0, ty = oy - fy0;
-    if (tx < 1e-4f && ty < 1e-4f) tx = ty = 0.0f;
-    const int c0 = min(x0 + x, W - 1);
-    const int dc = min(x0 + x + 1, W - 1) - c0;  // 1, or 0 at the right border
-    const float* base = img + (size_t)y0 * W + c0;
-    const int last = H - 1 - y0;                  // rows below y0 that exist
-    float top = __ldg(base), topr = __ldg(base + dc);
-    float ht = fmaf(tx, topr - top, top);
+// rows of both frames at once, A into the real and B into the imaginary part: each lane loads both
+// taps of every row itself (the right-hand tap is the next float, or the same one at the right image
+// border), with no shuffles and no conditional loads; the row below is carried to the next
+// iteration. The bilinear weights are applied as two linear interpolations with FMA (rounding differs
+// from the reference's weight sum by an ulp, far below the split-BF16 precision), in packed operations
+// for both frames; zero fractions make it an exact copy. The kernels wait on these loads more than on
+// anything else, and both frames' loads are in flight together (2048 x 2048 pair, 64 px pass 187 -> 161 us, 16 px 122 -> 112).
+template <int N>
+__device__ __forceinline__ void sample_rows(const float* __restrict__ img_a, const float* __restrict__ img_b, int H, int W,
+                                            float4 o, int x, float2 (&z)[N]) {
+    const PairSource s = pair_source(img_a, img_b, H, W, o, x);
+    float2 tx = s.tx, ty = s.ty;
+    if (s.copy_a) tx.x = ty.x = 0.0f;
+    if (s.copy_b) tx.y = ty.y = 0.0f;
+    auto lerp = [](float2 t, float2 u, float2 v) { return cfma2(t, csub(v, u), u); };
+    float2 ht = lerp(tx, make_float2(__ldg(s.a), __ldg(s.b)), make_float2(__ldg(s.a + s.right_a), __ldg(s.b + s.right_b)));
+    if (min(s.last_a, s.last_b) >= N && (s.right_a & s.right_b)) {  // all taps exist: pointers step by the pitch
+        const float *qa = s.a, *qb = s.b;
 #pragma unroll
-    for (int p = 0; p < N; ++p) {
-        const float* row = base + (size_t)min(p + 1, last) * W;
-        const float bot = __ldg(row), botr = __ldg(row + dc);
-        const float hb = fmaf(tx, botr - bot, bot);
-        const float v = fmaf(ty, hb - ht, ht);
-        if (IMAG) z[p].y = v; else z[p].x = v;
-        ht = hb;
+        for (int p = 0; p < N; ++p) {
+            qa += W;
+            qb += W;
+            const float2 hb = lerp(tx, make_float2(__ldg(qa), __ldg(qb)), make_float2(__ldg(qa + 1), __ldg(qb + 1)));
+            z[p] = lerp(ty, ht, hb);
+            ht = hb;
+        }
+    } else {
+#pragma unroll
+        for (int p = 0; p < N; ++p) {
+            const float* qa = s.a + (size_t)min(p + 1, s.last_a) * W;
+            const float* qb = s.b + (size_t)min(p + 1, s.last_b) * W;
+            const float2 hb =
+                lerp(tx, make_float2(__ldg(qa), __ldg(qb)), make_float2(__ldg(qa + s.right_a), __ldg(qb + s.right_b)));
+            z[p] = lerp(ty, ht, hb);
+            ht = hb;
+        }
     }
 }
 
@@ -310,27 +320,23 @@ __global__ void __launch_bounds__(TcCfg<N>::THREADS, TcCfg<N>::CTAS_PER_SM)
             sample_deformed<N>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, q, 0, 1, c_ramp<N>(),
                                SeparateProduct(prm.ncells), z);
         } else {
-            sample_rows<N, false>(prm.img_a, prm.H, prm.W, org.x, org.y, q, z);
-            sample_rows<N, true>(prm.img_b, prm.H, prm.W, org.z, org.w, q, z);
+            sample_rows<N>(prm.img_a, prm.img_b, prm.H, prm.W, org, q, z);
         }
         float2 e;
         {
             float2 s = make_float2(0.f, 0.f);
 #pragma unroll
             for (int p = 0; p < N; ++p) {
-                s.x += z[p].x;
-                s.y += z[p].y;
+                s = cadd(s, z[p]);
             }
             s = win_sum2<N>(s, red, i, wg);
             constexpr float inv = 1.0f / (float)(N * N);
-            const float ma = s.x * inv, mb = s.y * inv;
+            const float2 m = make_float2(s.x * inv, s.y * inv);  // inv is a power of two: exact
             e = make_float2(0.f, 0.f);
 #pragma unroll
             for (int p = 0; p < N; ++p) {
-                z[p].x = __fsub_rn(z[p].x, ma);
-                z[p].y = __fsub_rn(z[p].y, mb);
-                e.x += z[p].x * z[p].x;
-                e.y += z[p].y * z[p].y;
+                z[p] = csub(z[p], m);
+                e = cfma2(z[p], z[p], e);
             }
             e = win_sum2<N>(e, red, i, wg);
         }
