@@ -210,6 +210,15 @@ __device__ __forceinline__ void fix_stats_fast(long long sum1, long long sum2, f
     *std_out = __fmaf_rn(__fadd_rn(__fsub_rn(__fsub_rn(var.hi, p.hi), p.lo), var.lo), h, g);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Programmatic dependent launch: a kernel launched through launch_dependent (kernels.h) may start
+// while the kernel before it in the stream is finishing. Its threads call dependent_wait() before they
+// read or write anything another kernel touches (it returns once that kernel has completed and its
+// writes are visible; at once when the launch has no such predecessor), then let_dependents_start().
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_dependents_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 // Rust f32::clamp (NaN passes through).
 __device__ __forceinline__ float rclamp(float x, float lo, float hi) {
     if (x < lo) return lo;

@@ -280,6 +280,8 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
         if constexpr (C::DEFORM) s_ramp[i] = __fdiv_rn((float)i, (float)(N - 1));
     }
     __syncthreads();
+    dependent_wait();  // the tables above need nothing of the kernels before
+    let_dependents_start();
 
     const long long base_cell = ((long long)block * G + g) * WPG;
     float4 org[WPG];  // uniform shift: origins; deformed: (D(centre).x, D(centre).y, -, -)
@@ -860,8 +862,7 @@ cudaError_t launch_correlate_fused(const CorrParams* items, const int* kinds, in
         b.block_start[b.n] = (int)total;
         if (total > 0x7fffffffll) return cudaErrorInvalidValue;
         if (total > 0) {
-            correlate_fused_kernel<<<(unsigned)total, kFusedThreads, kFusedSmem, s>>>(b);
-            e = cudaGetLastError();
+            e = launch_dependent(correlate_fused_kernel, (unsigned)total, kFusedThreads, kFusedSmem, s, b);
             if (e != cudaSuccess) return e;
             if (launches) ++*launches;
         }
@@ -886,8 +887,7 @@ static cudaError_t launch_t(CorrBatch b, cudaStream_t s) {
     // Attribute setting is idempotent and per device; done on every launch for simplicity.
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)total, C::THREADS, C::SMEM, s>>>(b);
-    return cudaGetLastError();
+    return launch_dependent(kern, (unsigned)total, C::THREADS, C::SMEM, s, b);
 }
 
 bool corr_supported(int n) {

@@ -87,6 +87,8 @@ struct ValidateBatch {
 };
 
 __global__ void place_kernel(const __grid_constant__ PlaceBatch b) {
+    dependent_wait();
+    let_dependents_start();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= b.cell_start[b.n]) return;
     const int it = batch_item(b.cell_start, b.n, u);
@@ -152,8 +154,7 @@ cudaError_t launch_place_items(const PlaceParams* items, int count, cudaStream_t
         b.cell_start[b.n] = (int)total;
         if (total <= 0) continue;
         if (total > 0x7fffffffll) return cudaErrorInvalidValue;
-        place_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(b);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_dependent(place_kernel, (unsigned)((total + 255) / 256), 256, 0, s, b);
         if (e != cudaSuccess) return e;
         if (launches) ++*launches;
     }
@@ -271,6 +272,8 @@ __global__ void __launch_bounds__(kValidateThreads) validate_kernel(const __grid
     __shared__ float su[LY][LX], sv[LY][LX];
     __shared__ uint8_t s1[LY][LX], s2[MY][MX];
     __shared__ unsigned int s_count[5];
+    dependent_wait();
+    let_dependents_start();
     const int it = batch_item(b.tile_start, b.n, (int)blockIdx.x);
     const ValidateParams& p = b.item[it];
     const int tile = (int)blockIdx.x - b.tile_start[it], tiles_x = (p.nx + kTileX - 1) / kTileX;
@@ -388,11 +391,8 @@ cudaError_t launch_validate_items(const ValidateParams* items, int count, cudaSt
         b.tile_start[b.n] = (int)total;
         if (total <= 0) continue;
         if (total > 0x7fffffffll) return cudaErrorInvalidValue;
-        if (ty == 32)
-            validate_kernel<32><<<(unsigned)total, kValidateThreads, 0, s>>>(b);
-        else
-            validate_kernel<8><<<(unsigned)total, kValidateThreads, 0, s>>>(b);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_dependent(ty == 32 ? validate_kernel<32> : validate_kernel<8>, (unsigned)total,
+                                               kValidateThreads, 0, s, b);
         if (e != cudaSuccess) return e;
         if (launches) ++*launches;
     }
@@ -413,6 +413,8 @@ struct ExportBatch {
 constexpr int kExportThreads = 256, kExportCells = 4 * kExportThreads;
 
 __global__ void __launch_bounds__(kExportThreads) export_kernel(const __grid_constant__ ExportBatch b) {
+    dependent_wait();
+    let_dependents_start();
     const int it = batch_item(b.block_start, b.n, (int)blockIdx.x);
     const ExportItem& q = b.item[it];
     const int base = ((int)blockIdx.x - b.block_start[it]) * kExportCells;
@@ -451,8 +453,7 @@ cudaError_t launch_export_items(const ExportItem* items, int count, cudaStream_t
         b.block_start[b.n] = (int)total;
         if (total <= 0) continue;
         if (total > 0x7fffffffll) return cudaErrorInvalidValue;
-        export_kernel<<<(unsigned)total, kExportThreads, 0, s>>>(b);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_dependent(export_kernel, (unsigned)total, kExportThreads, 0, s, b);
         if (e != cudaSuccess) return e;
         if (launches) ++*launches;
     }

@@ -11,6 +11,24 @@ namespace pivb200 {
 // Sets the message piv_last_error returns on this host thread.
 void set_last_error(const char* msg);
 
+// Launches a kernel that calls dependent_wait() (common.cuh), allowed to start before the previous
+// kernel of the stream has ended: its launch, block scheduling and table set-up then overlap that
+// kernel's tail. A short chain is mostly such gaps (one-pass 512 x 512 pair, 6 kernels: 39.0 -> 34.6 us).
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // ----------------------------------------------------------------------------- correlation
 struct CorrParams {
     const float* img_a;

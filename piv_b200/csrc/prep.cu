@@ -56,6 +56,8 @@ __global__ void __launch_bounds__(kHistThreads) hist_kernel(const CodeT* __restr
     __shared__ bool last;
     for (int i = threadIdx.x; i < kBins; i += kHistThreads) h[i] = 0;
     __syncthreads();
+    dependent_wait();
+    let_dependents_start();
     constexpr bool kOneByte = sizeof(CodeT) == 1;  // level 1 alone, in the one coarse bin there is
     const unsigned int coarse = LEVEL && !kOneByte ? sel[0] : 0u;
     auto count = [&](unsigned int c) {
@@ -262,6 +264,8 @@ __device__ __forceinline__ float convert_codes(const CodeT* __restrict__ raw, lo
 template <typename CodeT>
 __global__ void convert_kernel(const CodeT* __restrict__ raw, long long n, const float* __restrict__ bg,
                                const unsigned int* clip, float* __restrict__ out, unsigned int* maxout) {
+    dependent_wait();
+    let_dependents_start();
     const float m = convert_codes(raw, n, bg, clip, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
                                   (long long)gridDim.x * blockDim.x);
     if (maxout) block_max_to(m, maxout);
@@ -280,6 +284,8 @@ struct ConvertBatch {
 
 template <typename CodeT>
 __global__ void convert_frames_kernel(const __grid_constant__ ConvertBatch b) {
+    dependent_wait();
+    let_dependents_start();
     const int f = (int)blockIdx.x / b.per;
     const long long tid = (long long)(blockIdx.x - f * b.per) * blockDim.x + threadIdx.x;
     convert_codes(static_cast<const CodeT*>(b.raw[f]), b.n, b.bg, nullptr, b.out[f], tid, (long long)b.per * blockDim.x);
@@ -287,6 +293,8 @@ __global__ void convert_frames_kernel(const __grid_constant__ ConvertBatch b) {
 
 __global__ void convert_f32_kernel(const float* __restrict__ raw, long long n, const float* __restrict__ bg,
                                    float* __restrict__ out, unsigned int* maxout) {
+    dependent_wait();
+    let_dependents_start();
     const FloatSamples src{raw, bg};
     float m = 0.0f;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -323,6 +331,8 @@ __global__ void __launch_bounds__(kStripThreads) integral_strip_kernel(const flo
                                                                        long long* __restrict__ sumsq,
                                                                        const unsigned int* maxbits, int* scales) {
     constexpr int R = kStripRows;
+    dependent_wait();
+    let_dependents_start();
     static_assert(2 * R == kStripWarps, "one warp scans the warp totals of each row of each table");
     const FixScale fs = fix_scale(__uint_as_float(*maxbits), (long long)H * W);
     const int y0 = blockIdx.x * R, rows = min(R, H - y0);
@@ -380,6 +390,8 @@ __global__ void __launch_bounds__(kStripThreads) integral_strip_kernel(const flo
 // Rows kStripRows, 2 kStripRows, ... of both tables become running sums down each column: 32
 // columns and 32 groups of strips per block.
 __global__ void __launch_bounds__(1024) integral_scan_kernel(int H, int W, long long* sum, long long* sumsq) {
+    dependent_wait();
+    let_dependents_start();
     const int strips = H / kStripRows;  // full strips; a last partial one has no row to update
     const int stride = W + 1;
     const int tx = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -421,6 +433,8 @@ template <typename Src, int RC>
 __global__ void blur_kernel(Src src, int H, int W, const BlurKernel k, float* __restrict__ out,
                             unsigned int* maxout) {
     extern __shared__ float sm[];
+    dependent_wait();
+    let_dependents_start();
     src.begin();
     const int R = RC > 0 ? RC : k.radius;
     const int TW = BT_X + 2 * R, TH = BT_Y + 2 * R;
@@ -480,6 +494,8 @@ template <int RC>
 __global__ void normalize_kernel(const float* __restrict__ src, int H, int W, int r_arg, float eps,
                                  const unsigned int* maxbits, float* __restrict__ out) {
     extern __shared__ long long smq[];
+    dependent_wait();
+    let_dependents_start();
     const int r = RC > 0 ? RC : r_arg;
     const int TW = NT_X + 2 * r, TH = NT_Y + 2 * r;
     // Row strides in 8-byte words are odd (QW, NT_HW), so 16 lanes on 16 consecutive rows of one
@@ -590,15 +606,13 @@ template <typename Src>
 static cudaError_t run_blur(dim3 grid, size_t sm, cudaStream_t s, const Src& src, int H, int W, const BlurKernel& k,
                             float* dst, unsigned int* mx) {
     if (k.radius == 3) {
-        blur_kernel<Src, 3><<<grid, kBlurThreads, sm, s>>>(src, H, W, k, dst, mx);
-        return cudaSuccess;
+        return launch_dependent(blur_kernel<Src, 3>, grid, kBlurThreads, sm, s, src, H, W, k, dst, mx);
     }
     if (sm > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(blur_kernel<Src, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
     }
-    blur_kernel<Src, 0><<<grid, kBlurThreads, sm, s>>>(src, H, W, k, dst, mx);
-    return cudaSuccess;
+    return launch_dependent(blur_kernel<Src, 0>, grid, kBlurThreads, sm, s, src, H, W, k, dst, mx);
 }
 
 static int grid_for(long long n) {
@@ -678,10 +692,11 @@ __global__ void table_to_fixed_kernel(unsigned long long* t, long long n, const 
 // The tables from `base` and its max |v| in *maxbits.
 static cudaError_t run_tables(const float* base, int H, int W, long long* sum, long long* sumsq, int* scales,
                               const unsigned int* maxbits, cudaStream_t s, int* launches) {
-    integral_strip_kernel<<<(H + kStripRows - 1) / kStripRows, kStripThreads, 0, s>>>(base, H, W, sum, sumsq, maxbits, scales);
-    integral_scan_kernel<<<(W + 1 + 31) / 32, 1024, 0, s>>>(H, W, sum, sumsq);
+    cudaError_t e = launch_dependent(integral_strip_kernel, (H + kStripRows - 1) / kStripRows, kStripThreads, 0, s, base, H, W,
+                                     sum, sumsq, maxbits, scales);
+    if (e == cudaSuccess) e = launch_dependent(integral_scan_kernel, (W + 1 + 31) / 32, 1024, 0, s, H, W, sum, sumsq);
     if (launches) *launches += 2;
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_stats(const float* base, int H, int W, long long* sum, long long* sumsq, int* scales,
@@ -740,13 +755,11 @@ cudaError_t launch_convert_frames(const void* const* raw, float* const* out, int
             b.out[i] = out[off + i];
         }
         b.bg = background;
+        cudaError_t e = cudaErrorInvalidValue;
         if (raw_type == RAW_U8)
-            convert_frames_kernel<uint8_t><<<(unsigned)(m * b.per), 256, 0, s>>>(b);
+            e = launch_dependent(convert_frames_kernel<uint8_t>, (unsigned)(m * b.per), 256, 0, s, b);
         else if (raw_type == RAW_U16)
-            convert_frames_kernel<uint16_t><<<(unsigned)(m * b.per), 256, 0, s>>>(b);
-        else
-            return cudaErrorInvalidValue;
-        const cudaError_t e = cudaGetLastError();
+            e = launch_dependent(convert_frames_kernel<uint16_t>, (unsigned)(m * b.per), 256, 0, s, b);
         if (e != cudaSuccess) return e;
         if (launches) ++*launches;
     }
@@ -755,7 +768,7 @@ cudaError_t launch_convert_frames(const void* const* raw, float* const* out, int
 
 cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches) {
     const long long n = (long long)p.H * p.W;
-    cudaError_t e;
+    cudaError_t e = cudaSuccess;
     int nl = 0;
     const unsigned int* clip = nullptr;
     if (p.clip_percentile_on && (p.raw_type == RAW_U8 || p.raw_type == RAW_U16)) {
@@ -768,11 +781,13 @@ cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches) {
         const int blocks = (int)std::min<long long>(grid_for(n), 148 * 2);
         if (p.raw_type == RAW_U16) {
             const uint16_t* raw = (const uint16_t*)p.raw;
-            hist_kernel<uint16_t, 0><<<blocks, kHistThreads, 0, s>>>(raw, n, p.hist, sel, target);
-            hist_kernel<uint16_t, 1><<<blocks, kHistThreads, 0, s>>>(raw, n, p.hist, sel, target);
+            e = launch_dependent(hist_kernel<uint16_t, 0>, blocks, kHistThreads, 0, s, raw, n, p.hist, sel, target);
+            if (e == cudaSuccess)
+                e = launch_dependent(hist_kernel<uint16_t, 1>, blocks, kHistThreads, 0, s, raw, n, p.hist, sel, target);
         } else {
-            hist_kernel<uint8_t, 1><<<blocks, kHistThreads, 0, s>>>((const uint8_t*)p.raw, n, p.hist, sel, target);
+            e = launch_dependent(hist_kernel<uint8_t, 1>, blocks, kHistThreads, 0, s, (const uint8_t*)p.raw, n, p.hist, sel, target);
         }
+        if (e != cudaSuccess) return e;
         nl += p.raw_type == RAW_U16 ? 2 : 1;
         clip = sel;
     }
@@ -792,15 +807,16 @@ cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches) {
     unsigned int* bmax = base_max ? p.maxbits : nullptr;
     if (!fused) switch (p.raw_type) {
         case RAW_U8:
-            convert_kernel<uint8_t><<<grid_for(n), 256, 0, s>>>((const uint8_t*)p.raw, n, p.background, clip, base, bmax);
+            e = launch_dependent(convert_kernel<uint8_t>, grid_for(n), 256, 0, s, (const uint8_t*)p.raw, n, p.background, clip, base, bmax);
             break;
         case RAW_U16:
-            convert_kernel<uint16_t><<<grid_for(n), 256, 0, s>>>((const uint16_t*)p.raw, n, p.background, clip, base, bmax);
+            e = launch_dependent(convert_kernel<uint16_t>, grid_for(n), 256, 0, s, (const uint16_t*)p.raw, n, p.background, clip, base, bmax);
             break;
         default:
-            convert_f32_kernel<<<grid_for(n), 256, 0, s>>>((const float*)p.raw, n, p.background, base, bmax);
+            e = launch_dependent(convert_f32_kernel, grid_for(n), 256, 0, s, (const float*)p.raw, n, p.background, base, bmax);
             break;
     }
+    if (e != cudaSuccess) return e;
     if (!fused) nl += 1;
     if (p.build_stats) {
         e = run_tables(base, p.H, p.W, p.sum, p.sumsq, p.scales, p.maxbits, s, &nl);
@@ -837,14 +853,15 @@ cudaError_t launch_prepare(const PrepParams& p, cudaStream_t s, int* launches) {
         const size_t sm = sizeof(long long) * (2 * (size_t)(NT_Y + 2 * r) * ((NT_X + 2 * r) | 1) + 2 * (size_t)(NT_Y + 2 * r) * NT_HW);
         dim3 grid((p.W + NT_X - 1) / NT_X, (p.H + NT_Y - 1) / NT_Y);
         if (r == 4) {  // the default radius: 37.9 KB of tile, under the 48 KB default
-            normalize_kernel<4><<<grid, kNormThreads, sm, s>>>(cur, p.H, p.W, r, p.normalize_eps, mx, p.image);
+            e = launch_dependent(normalize_kernel<4>, grid, kNormThreads, sm, s, cur, p.H, p.W, r, p.normalize_eps, mx, p.image);
         } else {
             if (sm > 48 * 1024) {
                 e = cudaFuncSetAttribute(normalize_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
                 if (e != cudaSuccess) return e;
             }
-            normalize_kernel<0><<<grid, kNormThreads, sm, s>>>(cur, p.H, p.W, r, p.normalize_eps, mx, p.image);
+            e = launch_dependent(normalize_kernel<0>, grid, kNormThreads, sm, s, cur, p.H, p.W, r, p.normalize_eps, mx, p.image);
         }
+        if (e != cudaSuccess) return e;
         nl += 1;
         cur = p.image;
     }
