@@ -441,7 +441,7 @@ int run_passes_eager(PivAnalyzer* an, const PivFrame* const* a, const PivFrame* 
             pp.zero_counts = i == 0 ? an->d_counts + 8 * (size_t)k : nullptr;
             cps[k] = CorrParams{a[k]->image, b[k]->image, (int)H, (int)W, pb.origins, pb.status, (int)pb.cells,
                                 pb.raw_dx, pb.raw_dy, pb.raw_ppr, pb.raw_flags, pp.corners, (int)pb.grid.x0,
-                                (int)pb.grid.y0, (int)pb.grid.step, (int)pb.grid.nx};
+                                (int)pb.grid.y0, (int)pb.grid.step, (int)pb.grid.nx, i == 0};
             vps[k] = ValidateParams{(int)pb.grid.nx, (int)pb.grid.ny, pb.raw_dx, pb.raw_dy, pb.raw_ppr, pb.raw_flags,
                                     pb.dx, pb.dy, pb.flags, (float)an->windows[0] / 2.0f, an->ppr_threshold,
                                     an->median_threshold, an->median_eps, an->replace,
@@ -2307,7 +2307,7 @@ void PivServer::launch_step(std::vector<Request*>& work) {
         cps[{(int)pb.grid.window, kind}].push_back(
             CorrParams{r->fa.image, r->fb.image, (int)r->H, (int)r->W, pb.origins, pb.status, (int)pb.cells, pb.raw_dx,
                        pb.raw_dy, pb.raw_ppr, pb.raw_flags, pp.corners, (int)pb.grid.x0, (int)pb.grid.y0,
-                       (int)pb.grid.step, (int)pb.grid.nx});
+                       (int)pb.grid.step, (int)pb.grid.nx, i == 0});
         vps.push_back(ValidateParams{(int)pb.grid.nx, (int)pb.grid.ny, pb.raw_dx, pb.raw_dy, pb.raw_ppr, pb.raw_flags, pb.dx,
                                      pb.dy, pb.flags, (float)r->cfg.windows[0] / 2.0f, r->cfg.ppr_threshold,
                                      r->cfg.median_threshold, r->cfg.median_eps, r->cfg.replace,

@@ -39,15 +39,25 @@ namespace pivb200 {
 // single windows, groups per CTA G, minimum resident CTAs per SM (register cap).
 // G and MINB only change the launch geometry, never the arithmetic; N, T and PAIR fix the FFT
 // decomposition and therefore the rounding of the results.
-template <int N_, int T_, bool PAIR_, int G_, int MINB_, bool DEFORM_ = false>
+template <int N_, int T_, bool PAIR_, int G_, int MINB_, bool DEFORM_ = false, bool COPY_ = false>
 struct CorrCfg {
     static constexpr int N = N_, T = T_, G = G_, MINB = MINB_;
-    static constexpr bool PAIR = PAIR_, DEFORM = DEFORM_;
+    static constexpr bool PAIR = PAIR_, DEFORM = DEFORM_, COPY = COPY_;  // COPY: whole-pixel windows only
     // 32 and 64 px windows (and one-lane lines, where the layouts are the same) run the column pass
     // of the forward FFT from the block layout (lane t holds rows P*rev(t) + p; bit-reversed blocks
     // in, lane t ends with the frequency rows t + T*k), the others from interleaved rows (t + T*p).
     // The two round differently, so a size keeps its own.
     static constexpr bool BLOCK = T_ == 1 || N_ == 32 || N_ == 64;
+    // Lines of several lanes: a warp that samples T blocks of rows of 32/T columns touches T lines of
+    // the image per load (4.7 L1 wavefronts each on four lanes, 2.6 on two), a third of the data pipe's
+    // work at 64 px. Instead a warp samples 32 columns of one block, and the planes pass the samples on
+    // to the lanes that transform them. Interpolated passes of a 2048 x 2048 pair, before and after: 64
+    // px 511 -> 457 us, 128 px 627 -> 568; 2400 x 2400: 48 px 776 -> 755, 24 px 643 -> 615. At 32 px the
+    // exchange costs what it saves. Whole-pixel windows have one load per sample, and the sizes that
+    // want rows t + T*p lose by it (96 px 681 -> 765 us); every first pass is of that kind and runs
+    // kernels of its own (COPY), which need no registers for the interpolation either (96 px 682 -> 649
+    // us, 24 px 101 -> 95, the 128 px pass of a 4096 x 4096 pair 2.19 -> 2.16 ms).
+    static constexpr bool EXCHANGE = T_ > 1 && N_ != 32;
     static constexpr int P = N / T;
     static constexpr int NT = N * T;
     static constexpr int THREADS = G * NT;
@@ -83,9 +93,9 @@ struct CorrCfg {
     __host__ __device__ static constexpr int AF(int row, int col) {
         return (BLOCK && T == 2) ? row * N + ((col + 2 * (((row >> 1) & 3) + 4 * (row & 1))) & (N - 1)) : A(row, col);
     }
-    // The exchange of sampled rows (stored as rows P*rev(t) + p, read as rows t + T*p, by the lanes of
-    // 16/T columns per half-warp): A on four lanes; on two (24 px), rows of 32 rotated by 8 where the
-    // row's parity and half differ, again 16 distinct bank pairs either way.
+    // The exchange of sampled rows (stored by consecutive columns of a row, read as rows t + T*p or
+    // P*rev(t) + p by the lanes of 16/T columns per half-warp): A on four lanes; on two, rows of 32
+    // rotated by 8 where the row's parity and half differ, 16 distinct bank pairs either way.
     __host__ __device__ static constexpr int AX(int row, int col) {
         return T == 2 ? row * 32 + ((col + 8 * ((row & 1) ^ (row >= P ? 1 : 0))) & 31) : A(row, col);
     }
@@ -299,9 +309,9 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
         ok[wi] = active && prm.status[cell] != 0;
     }
     const SeparateProduct mul(prm.ncells);
-    if constexpr (C::DEFORM) {
-#pragma unroll
-        for (int wi = 0; wi < WPG; ++wi) {
+    // Window wi's column x, rows r0 .. r0 + P - 1, of both frames.
+    auto sample = [&](int wi, int x, int r0, float2 (&z)[P]) {
+        if constexpr (C::DEFORM) {
             const long long cell = base_cell + wi;
             const bool active = cell < prm.ncells;
             const int ci = active ? (int)cell : 0;
@@ -312,43 +322,42 @@ __device__ __forceinline__ void correlate_body(const CorrParams& prm, int block,
             const int gy = min(prm.gy0 + (ci / prm.gnx) * prm.gstep, max(prm.H - N - 1, 0));
             org[wi] = make_float4(corner_blend(k0.x, k0.z, k1.x, k1.z, 0.5f, 0.5f),
                                   corner_blend(k0.y, k0.w, k1.y, k1.w, 0.5f, 0.5f), 0.f, 0.f);
-            if (wi == 0) {
-                sample_deformed<N>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, line, C::BLOCK ? P * rt : t,
-                                   C::BLOCK ? 1 : T, s_ramp, mul, z0);
-            } else if constexpr (PAIR) {
-                sample_deformed<N>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, line, C::BLOCK ? P * rt : t,
-                                   C::BLOCK ? 1 : T, s_ramp, mul, z1);
+            sample_deformed<N>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, x, r0, s_ramp, mul, z);
+        } else {
+            const PairSource p = pair_source(prm.img_a, prm.img_b, prm.H, prm.W, org[wi], x);
+            if (C::COPY || (p.copy_a && p.copy_b)) copy_rows(p, prm.W, r0, 1, z); else stream_rows<N>(p, prm.W, r0, mul, z);
+        }
+    };
+    if constexpr (C::COPY && N != 64) {  // 64 px: 425 us through the exchange, 444 straight
+        const int first = C::BLOCK ? P * rt : t, step = C::BLOCK ? 1 : T;
+        copy_rows(pair_source(prm.img_a, prm.img_b, prm.H, prm.W, org[0], line), prm.W, first, step, z0);
+        if constexpr (PAIR)
+            copy_rows(pair_source(prm.img_a, prm.img_b, prm.H, prm.W, org[1], line), prm.W, first, step, z1);
+    } else if constexpr (!C::EXCHANGE) {
+        sample(0, line, P * rt, z0);
+        if constexpr (PAIR) sample(1, line, P * rt, z1);
+    } else {
+        // Neighbouring threads sample neighbouring columns of one block of rows, so a warp's loads read
+        // whole lines; the planes then hand each lane its own rows (rows t + T*p, or the block P*rev(t)).
+        // They are not written again before the group barriers of the sums below.
+        const int x = gt % N, r0 = P * (gt / N);
+        {
+            float2 v[P];
+            sample(0, x, r0, v);
+#pragma unroll
+            for (int p = 0; p < P; ++p) plane0[C::AX(r0 + p, x)] = v[p];
+            if constexpr (PAIR) {
+                sample(1, x, r0, v);
+#pragma unroll
+                for (int p = 0; p < P; ++p) reinterpret_cast<float2*>(plane1_raw)[C::AX(r0 + p, x)] = v[p];
             }
         }
-    } else {
-        const PairSource p0 = pair_source(prm.img_a, prm.img_b, prm.H, prm.W, org[0], line);
-        const PairSource p1 = pair_source(prm.img_a, prm.img_b, prm.H, prm.W, org[WPG - 1], line);
-        if constexpr (C::BLOCK) {
-            if (p0.copy_a && p0.copy_b) copy_rows(p0, prm.W, P * rt, 1, z0); else stream_rows<N>(p0, prm.W, P * rt, mul, z0);
-            if constexpr (PAIR) {
-                if (p1.copy_a && p1.copy_b) copy_rows(p1, prm.W, P * rt, 1, z1); else stream_rows<N>(p1, prm.W, P * rt, mul, z1);
-            }
-        } else if (p0.copy_a && p0.copy_b && p1.copy_a && p1.copy_b) {  // the same for the whole group
-            copy_rows(p0, prm.W, t, T, z0);
-            if constexpr (PAIR) copy_rows(p1, prm.W, t, T, z1);
-        } else {
-            // streamed block rows, then the T lanes of a column exchange them for rows t + T*p; the planes
-            // are not written again before the group barriers of the sums below
-            const unsigned line_lanes = ((1u << T) - 1u) << ((threadIdx.x & 31) - t);
-            stream_rows<N>(p0, prm.W, P * rt, mul, z0);
-            if constexpr (PAIR) stream_rows<N>(p1, prm.W, P * rt, mul, z1);
+        group_sync<C>(g);
 #pragma unroll
-            for (int p = 0; p < P; ++p) {
-                plane0[C::AX(P * rt + p, line)] = z0[p];
-                if constexpr (PAIR) reinterpret_cast<float2*>(plane1_raw)[C::AX(P * rt + p, line)] = z1[p];
-            }
-            __syncwarp(line_lanes);
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                z0[p] = plane0[C::AX(t + T * p, line)];
-                if constexpr (PAIR) z1[p] = reinterpret_cast<float2*>(plane1_raw)[C::AX(t + T * p, line)];
-            }
-            __syncwarp(line_lanes);
+        for (int p = 0; p < P; ++p) {
+            const int row = C::BLOCK ? P * rt + p : t + T * p;
+            z0[p] = plane0[C::AX(row, line)];
+            if constexpr (PAIR) z1[p] = reinterpret_cast<float2*>(plane1_raw)[C::AX(row, line)];
         }
     }
     {
@@ -908,20 +917,24 @@ bool corr_supported(int n) {
 struct CorrVariant {
     const char* name;
     cudaError_t (*launch)(CorrBatch, cudaStream_t);
+    cudaError_t (*launch_whole)(CorrBatch, cudaStream_t);  // all items whole-pixel windows
 };
 
-#define PIV_V(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB, &launch_t<CorrCfg<N, T, PR, G, MB>>}
-static const CorrVariant kV8[] = {PIV_V(8, 1, true, 16, 6), PIV_V(8, 1, true, 32, 3), PIV_V(8, 1, true, 32, 4)};
-static const CorrVariant kV12[] = {PIV_V(12, 1, true, 16, 4), PIV_V(12, 1, true, 16, 3), PIV_V(12, 1, true, 8, 6)};
-static const CorrVariant kV16[] = {PIV_V(16, 1, true, 16, 2), PIV_V(16, 1, true, 8, 4), PIV_V(16, 1, true, 8, 5)};
-static const CorrVariant kV24[] = {PIV_V(24, 2, true, 2, 6), PIV_V(24, 2, true, 4, 3), PIV_V(24, 2, true, 2, 4)};
-static const CorrVariant kV32[] = {PIV_V(32, 2, true, 4, 2), PIV_V(32, 2, true, 2, 4), PIV_V(32, 2, true, 1, 8)};
-static const CorrVariant kV48[] = {PIV_V(48, 4, true, 1, 3), PIV_V(48, 4, true, 1, 2)};
-static const CorrVariant kV64[] = {PIV_V(64, 4, true, 1, 2), PIV_V(64, 4, true, 1, 1)};
-static const CorrVariant kV96[] = {PIV_V(96, 4, true, 1, 1)};
-static const CorrVariant kV128[] = {PIV_V(128, 4, false, 1, 1)};
+#define PIV_V(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB, &launch_t<CorrCfg<N, T, PR, G, MB>>, &launch_t<CorrCfg<N, T, PR, G, MB>>}
+// the default variants have a kernel of their own for whole-pixel windows
+#define PIV_W(N, T, PR, G, MB, CG, CMB) \
+    {#N "/T" #T "/G" #G "/B" #MB, &launch_t<CorrCfg<N, T, PR, G, MB>>, &launch_t<CorrCfg<N, T, PR, CG, CMB, false, true>>}
+static const CorrVariant kV8[] = {PIV_W(8, 1, true, 16, 6, 16, 6), PIV_V(8, 1, true, 32, 3), PIV_V(8, 1, true, 32, 4)};
+static const CorrVariant kV12[] = {PIV_W(12, 1, true, 16, 4, 16, 4), PIV_V(12, 1, true, 16, 3), PIV_V(12, 1, true, 8, 6)};
+static const CorrVariant kV16[] = {PIV_W(16, 1, true, 16, 2, 16, 2), PIV_V(16, 1, true, 8, 4), PIV_V(16, 1, true, 8, 5)};
+static const CorrVariant kV24[] = {PIV_W(24, 2, true, 2, 6, 2, 6), PIV_V(24, 2, true, 4, 3), PIV_V(24, 2, true, 2, 4)};
+static const CorrVariant kV32[] = {PIV_W(32, 2, true, 4, 2, 4, 2), PIV_V(32, 2, true, 2, 4), PIV_V(32, 2, true, 1, 8)};
+static const CorrVariant kV48[] = {PIV_W(48, 4, true, 1, 3, 1, 3), PIV_V(48, 4, true, 1, 2)};
+static const CorrVariant kV64[] = {PIV_W(64, 4, true, 1, 2, 1, 2), PIV_V(64, 4, true, 1, 1)};
+static const CorrVariant kV96[] = {PIV_W(96, 4, true, 1, 1, 1, 1)};
+static const CorrVariant kV128[] = {PIV_W(128, 4, false, 1, 1, 1, 1)};
 // Deformed-window variants: the same FFT decomposition per size, the deformed sampler.
-#define PIV_D(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB "/deform", &launch_t<CorrCfg<N, T, PR, G, MB, true>>}
+#define PIV_D(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB "/deform", &launch_t<CorrCfg<N, T, PR, G, MB, true>>, nullptr}
 static const CorrVariant kD8[] = {PIV_D(8, 1, true, 32, 3)};
 static const CorrVariant kD12[] = {PIV_D(12, 1, true, 16, 3)};
 static const CorrVariant kD16[] = {PIV_D(16, 1, true, 16, 2), PIV_D(16, 1, true, 8, 4)};
@@ -932,6 +945,7 @@ static const CorrVariant kD64[] = {PIV_D(64, 4, true, 1, 2)};
 static const CorrVariant kD96[] = {PIV_D(96, 4, true, 1, 1)};
 static const CorrVariant kD128[] = {PIV_D(128, 4, false, 1, 1)};
 #undef PIV_D
+#undef PIV_W
 #undef PIV_V
 
 static const CorrVariant* variants(int n, bool deform, int* count) {
@@ -982,8 +996,12 @@ cudaError_t launch_correlate_items(int n, int v, const CorrParams* items, int co
     for (int off = 0; off < count; off += kMaxBatch) {
         CorrBatch b;
         b.n = count - off < kMaxBatch ? count - off : kMaxBatch;
-        for (int i = 0; i < b.n; ++i) b.item[i] = items[off + i];
-        const cudaError_t e = vs[v].launch(b, s);
+        bool whole = !deform;
+        for (int i = 0; i < b.n; ++i) {
+            b.item[i] = items[off + i];
+            whole = whole && items[off + i].whole_pixels;
+        }
+        const cudaError_t e = whole ? vs[v].launch_whole(b, s) : vs[v].launch(b, s);
         if (e != cudaSuccess) return e;
         if (launches) ++*launches;
     }

@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(TcCfg<N>::THREADS, TcCfg<N>::CTAS_PER_SM)
             const int gy = min(prm.gy0 + (ci / prm.gnx) * prm.gstep, max(prm.H - N - 1, 0));
             org = make_float4(corner_blend(k0.x, k0.z, k1.x, k1.z, 0.5f, 0.5f),
                               corner_blend(k0.y, k0.w, k1.y, k1.w, 0.5f, 0.5f), 0.f, 0.f);
-            sample_deformed<N>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, q, 0, 1, c_ramp<N>(),
+            sample_deformed<N>(prm.img_a, prm.img_b, prm.H, prm.W, gx, gy, k0, k1, q, 0, c_ramp<N>(),
                                SeparateProduct(prm.ncells), z);
         } else {
             sample_rows<N>(prm.img_a, prm.img_b, prm.H, prm.W, org, q, z);

@@ -46,6 +46,8 @@ struct CorrParams {
     // dy11), and the pass grid that gives each cell's undeformed position.
     const float4* corners;
     int gx0, gy0, gstep, gnx;
+    // 1: every origin is a whole pixel in both frames (a pass without a predictor places them so)
+    int whole_pixels;
 };
 
 // Kernels take a batch of independent work items (pairs, passes or requests, of any sizes) by

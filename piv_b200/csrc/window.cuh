@@ -54,12 +54,23 @@ __device__ __forceinline__ PairSource pair_source(const float* __restrict__ img_
     return s;
 }
 
-// Copies rows first + step*p (both frames whole-pixel windows).
+// Copies rows first + step*p of whole-pixel windows. (With an address computed for every load, all of
+// them ahead of the loads, the registers spill.)
 template <int P>
 __device__ __forceinline__ void copy_rows(const PairSource& s, int W, int first, int step, float2 (&z)[P]) {
+    if (min(s.last_a, s.last_b) >= first + step * (P - 1)) {  // all rows exist: pointers step
+        const float *qa = s.a + first * W, *qb = s.b + first * W;
 #pragma unroll
-    for (int p = 0; p < P; ++p)
-        z[p] = make_float2(__ldg(s.a + min(first + step * p, s.last_a) * W), __ldg(s.b + min(first + step * p, s.last_b) * W));
+        for (int p = 0; p < P; ++p) {
+            z[p] = make_float2(__ldg(qa), __ldg(qb));
+            qa += step * W;
+            qb += step * W;
+        }
+    } else {
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            z[p] = make_float2(__ldg(s.a + min(first + step * p, s.last_a) * W), __ldg(s.b + min(first + step * p, s.last_b) * W));
+    }
 }
 
 // Samples the P consecutive rows from row r0 of the lane's column: the lane streams down them
@@ -108,8 +119,8 @@ __device__ __forceinline__ void stream_rows(PairSource s, int W, int r0, const S
     } else {
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            qa = s.a + min(r0 + p + 1, s.last_a) * W;
-            qb = s.b + min(r0 + p + 1, s.last_b) * W;
+            qa += r0 + p < s.last_a ? W : 0;
+            qb += r0 + p < s.last_b ? W : 0;
             const float2 bl = make_float2(__ldg(qa), __ldg(qb)),
                          br = make_float2(__ldg(qa + s.right_a), __ldg(qb + s.right_b));
             z[p] = blend(tl, tr, bl, br);
@@ -179,14 +190,15 @@ __device__ __forceinline__ float2 bilinear_inside(const float* __restrict__ img_
     return cadd(s, mul(cmul2(tx, ty), make_float2(__ldg(a + W + 1), __ldg(b + W + 1))));
 }
 
-// The lane fills z[p] = (A, B) at column x, row first + step*p.
+// The lane fills z[p] = (A, B) at column x, row r0 + p.
 template <int N, int P>
 __device__ __forceinline__ void sample_deformed(const float* __restrict__ img_a, const float* __restrict__ img_b, int H,
-                                                int W, int x0, int y0, float4 k0, float4 k1, int x, int first, int step,
+                                                int W, int x0, int y0, float4 k0, float4 k1, int x, int r0,
                                                 const float* s_ramp, const SeparateProduct& mul, float2 (&z)[P]) {
     const float u = s_ramp[x], ou = __fsub_rn(1.0f, u);
     const float2 d00 = make_float2(k0.x, k0.y), d10 = make_float2(k0.z, k0.w);
     const float2 d01 = make_float2(k1.x, k1.y), d11 = make_float2(k1.z, k1.w);
+    const float yf = (float)(y0 + r0);
     const float2 x2 = splat((float)(x0 + x)), sign = make_float2(-1.0f, 1.0f);
     // 0.5 |corner| bounds 0.5 |D| up to rounding; one pixel of margin covers that. (fmaxf drops a NaN,
     // so finite corners are asked for explicitly: every tap has to lie inside.)
@@ -206,15 +218,15 @@ __device__ __forceinline__ void sample_deformed(const float* __restrict__ img_a,
     if (inside) {
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            const float2 h = half(s_ramp[first + step * p]);
+            const float2 h = half(s_ramp[r0 + p]);
             z[p] = bilinear_inside(img_a, img_b, W, cfma2(splat(h.x), sign, x2),
-                                   cfma2(splat(h.y), sign, splat((float)(y0 + first + step * p))), mul);
+                                   cfma2(splat(h.y), sign, splat(__fadd_rn(yf, (float)p))), mul);
         }
     } else {
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            const float2 h = half(s_ramp[first + step * p]);
-            const float2 px = cfma2(splat(h.x), sign, x2), py = cfma2(splat(h.y), sign, splat((float)(y0 + first + step * p)));
+            const float2 h = half(s_ramp[r0 + p]);
+            const float2 px = cfma2(splat(h.x), sign, x2), py = cfma2(splat(h.y), sign, splat(__fadd_rn(yf, (float)p)));
             z[p] = make_float2(bilinear_clamped(img_a, H, W, px.x, py.x), bilinear_clamped(img_b, H, W, px.y, py.y));
         }
     }
