@@ -71,11 +71,13 @@ GridP to_gp(const PivGridC& g) {
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Device blocks of destroyed frames and of the blocking stage calls, kept for the next ones: a
-// program that makes frames for every pair spent more time in cudaMalloc and cudaFree than in the
-// analysis (1024 x 768 pair, host to host: 1.55 ms and more, 0.32 ms with the blocks kept). A block comes here only when no work can be using it (its giver has waited for the device or for its
-// stream). At most kKeptBytes are kept per device, in no one's name; they go back to the device when
-// an allocation fails and when the device's last analyzer is destroyed.
+// Device blocks of destroyed frames, of analyzers' workspaces and of the blocking stage calls, kept for
+// the next ones: a program that makes frames for every pair spent more time in cudaMalloc and cudaFree
+// than in the analysis (1024 x 768 pair, host to host: 1.55 ms and more, 0.30 ms with the blocks kept;
+// the first pass of a new analyzer on a 1024 x 1024 pair 0.70 -> 0.26 ms). A block comes here only when
+// no work can be using it (its giver has waited for the device or for its stream). At most kKeptBytes
+// are kept per device, in no one's name; they go back to the device when an allocation fails and when
+// the device's last analyzer is destroyed.
 constexpr size_t kKeptBytes = (size_t)256 << 20;
 struct KeptBlocks {
     std::multimap<size_t, void*> free;
@@ -203,6 +205,7 @@ struct PivAnalyzer {
     int K = 0;                                // pairs the workspace holds
     std::vector<std::vector<PassBuf>> pairs;  // [pair][pass]
     void* arena = nullptr;
+    size_t arena_bytes = 0;
     unsigned long long* d_counts = nullptr;
     long long launches = 0;
     // stage timing: per pass, pending (start, end) event pairs and the events to reuse
@@ -323,7 +326,8 @@ int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
     if (an->arena && an->H == H && an->W == W && an->K >= K) return PIV_OK;
     if (an->arena) {
         CUDA_TRY(cudaStreamSynchronize(an->cur));
-        CUDA_TRY(cudaFree(an->arena));
+        CUDA_TRY(cudaDeviceSynchronize());  // earlier calls may have run on other streams
+        give_block(an->device, an->arena, an->arena_bytes);
         an->arena = nullptr;
     }
     an->pairs.clear();
@@ -342,7 +346,8 @@ int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
         proto.push_back(pb);
     }
     const size_t total = align256(sizeof(unsigned long long) * 8 * (size_t)K) + per_pair * (size_t)K;
-    CUDA_TRY(device_malloc(&an->arena, total));
+    CUDA_TRY(take_block(&an->arena, total));
+    an->arena_bytes = total;
     char* p = (char*)an->arena;
     auto take = [&](size_t bytes) {
         void* r = p;
@@ -794,7 +799,12 @@ void piv_analyzer_destroy(PivAnalyzer* an) {
         cudaDeviceSynchronize();  // a replay may still run on a caller's stream
         cudaGraphExecDestroy(an->gexec);
     }
-    if (an->arena) cudaFree(an->arena);
+    if (an->arena) {
+        if (cudaDeviceSynchronize() == cudaSuccess)
+            give_block(an->device, an->arena, an->arena_bytes);
+        else
+            cudaFree(an->arena);
+    }
     if (an->own) cudaStreamDestroy(an->own);
     if (an->counted) count_analyzer(an->device, -1);
     delete an;
