@@ -217,7 +217,7 @@ struct PivAnalyzer {
     int variant[2][129] = {};
     // with tensor cores allowed: window sizes where the autotuner found the FP32 kernel faster
     bool fp32_faster[2][129] = {};  // [uniform / deformed windows][window]
-    // launch choices change (autotune, variant pinning): cached pass graphs are stale
+    // launch choices (autotune, variant pinning) or the workspace change: cached pass graphs are stale
     uint64_t epoch = 0;
     // the passes of the last repeated call, as a CUDA graph replayed while its key holds
     cudaGraphExec_t gexec = nullptr;
@@ -348,6 +348,7 @@ int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
     const size_t total = align256(sizeof(unsigned long long) * 8 * (size_t)K) + per_pair * (size_t)K;
     CUDA_TRY(take_block(&an->arena, total));
     an->arena_bytes = total;
+    ++an->epoch;  // the block may have the old one's address, but the layout depends on K, H and W
     char* p = (char*)an->arena;
     auto take = [&](size_t bytes) {
         void* r = p;
