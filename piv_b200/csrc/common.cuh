@@ -215,6 +215,12 @@ __device__ __forceinline__ void fix_stats_fast(long long sum1, long long sum2, f
 // while the kernel before it in the stream is finishing. Its threads call dependent_wait() before they
 // read or write anything another kernel touches (it returns once that kernel has completed and its
 // writes are visible; at once when the launch has no such predecessor), then let_dependents_start().
+// The kernel before may still write while this one is resident, so nothing it touches counts as
+// read-only here: such data is read through plain pointers, never through __ldg or a const
+// __restrict__ argument (the compiler may move those loads above the wait, and their path need not be
+// coherent). What was written by kernels further back is complete before this kernel starts, because
+// the one in between has waited for it; the correlation kernels read the frames through __ldg on that
+// ground (a placement or a copy always lies between them and the preparation).
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_dependents_start() { asm volatile("griddepcontrol.launch_dependents;"); }

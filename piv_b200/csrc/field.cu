@@ -19,7 +19,7 @@ __device__ __forceinline__ float grid_center(int origin0, int i, int step, int w
 }
 
 // VectorField::sample (field.rs:56-81).
-__device__ float2 sample_predictor(const float* __restrict__ dx, const float* __restrict__ dy, const GridP& g, float x,
+__device__ float2 sample_predictor(const float* dx, const float* dy, const GridP& g, float x,
                                    float y) {
     const float fx = rclamp(__fdiv_rn(__fsub_rn(x, grid_center(g.x0, 0, g.step, g.window)), (float)g.step), 0.0f,
                             (float)(g.nx - 1));

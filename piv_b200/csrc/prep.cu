@@ -47,7 +47,7 @@ struct BlurKernel {
 constexpr int kHistThreads = 256;
 
 template <typename CodeT, int LEVEL>
-__global__ void __launch_bounds__(kHistThreads) hist_kernel(const CodeT* __restrict__ raw, long long n, unsigned int* hist,
+__global__ void __launch_bounds__(kHistThreads) hist_kernel(const CodeT* raw, long long n, unsigned int* hist,
                                                             unsigned int* sel, unsigned long long target) {
     constexpr int kShift = 4;  // level 0 counts bins of code / 2^kShift
     constexpr int kBins = LEVEL == 0 ? 65536 >> kShift : 256;
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kHistThreads) hist_kernel(const CodeT* __restr
                 uint4 w;
                 CodeT c[V];
             } u;
-            u.w = __ldg(reinterpret_cast<const uint4*>(raw) + j);
+            u.w = reinterpret_cast<const uint4*>(raw)[j];
 #pragma unroll
             for (int k = 0; k < V; ++k) count(u.c[k]);
         }
@@ -220,8 +220,8 @@ __global__ void maxabs_kernel(const float* __restrict__ v, long long n, unsigned
 // also folds max |value| into it (the scale of the fixed-point sums), which saves a pass over the
 // frame. Launched with 256 threads.
 template <typename CodeT>
-__device__ __forceinline__ float convert_codes(const CodeT* __restrict__ raw, long long n, const float* __restrict__ bg,
-                                               const unsigned int* clip, float* __restrict__ out, long long tid,
+__device__ __forceinline__ float convert_codes(const CodeT* raw, long long n, const float* bg,
+                                               const unsigned int* clip, float* out, long long tid,
                                                long long stride) {
     constexpr int V = 16 / (int)sizeof(CodeT);
     CodeSamples<CodeT> src{raw, bg, clip, 0u, 0.0f, 0.0f};
@@ -242,11 +242,11 @@ __device__ __forceinline__ float convert_codes(const CodeT* __restrict__ raw, lo
                 uint4 w;
                 CodeT c[V];
             } u;
-            u.w = __ldg(reinterpret_cast<const uint4*>(raw) + j);
+            u.w = reinterpret_cast<const uint4*>(raw)[j];
 #pragma unroll
             for (int k = 0; k < V; k += 4) {
                 float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (bg) b = __ldg(reinterpret_cast<const float4*>(bg + j * V + k));
+                if (bg) b = *reinterpret_cast<const float4*>(bg + j * V + k);
                 float4 o;
                 o.x = value(u.c[k], b.x);
                 o.y = value(u.c[k + 1], b.y);
@@ -262,8 +262,8 @@ __device__ __forceinline__ float convert_codes(const CodeT* __restrict__ raw, lo
 }
 
 template <typename CodeT>
-__global__ void convert_kernel(const CodeT* __restrict__ raw, long long n, const float* __restrict__ bg,
-                               const unsigned int* clip, float* __restrict__ out, unsigned int* maxout) {
+__global__ void convert_kernel(const CodeT* raw, long long n, const float* bg,
+                               const unsigned int* clip, float* out, unsigned int* maxout) {
     dependent_wait();
     let_dependents_start();
     const float m = convert_codes(raw, n, bg, clip, out, (long long)blockIdx.x * blockDim.x + threadIdx.x,
@@ -291,8 +291,8 @@ __global__ void convert_frames_kernel(const __grid_constant__ ConvertBatch b) {
     convert_codes(static_cast<const CodeT*>(b.raw[f]), b.n, b.bg, nullptr, b.out[f], tid, (long long)b.per * blockDim.x);
 }
 
-__global__ void convert_f32_kernel(const float* __restrict__ raw, long long n, const float* __restrict__ bg,
-                                   float* __restrict__ out, unsigned int* maxout) {
+__global__ void convert_f32_kernel(const float* raw, long long n, const float* bg,
+                                   float* out, unsigned int* maxout) {
     dependent_wait();
     let_dependents_start();
     const FloatSamples src{raw, bg};
@@ -326,9 +326,9 @@ __device__ __forceinline__ long long warp_scan(long long v, int lane) {
     return v;
 }
 
-__global__ void __launch_bounds__(kStripThreads) integral_strip_kernel(const float* __restrict__ v, int H, int W,
-                                                                       long long* __restrict__ sum,
-                                                                       long long* __restrict__ sumsq,
+__global__ void __launch_bounds__(kStripThreads) integral_strip_kernel(const float* v, int H, int W,
+                                                                       long long* sum,
+                                                                       long long* sumsq,
                                                                        const unsigned int* maxbits, int* scales) {
     constexpr int R = kStripRows;
     dependent_wait();
@@ -430,7 +430,7 @@ constexpr int kBlurThreads = 256;  // the blur's launch width; its loops stride 
 // RC > 0 fixes the radius at compile time (the taps unroll; the summation order is unchanged);
 // RC = 0 takes it from k.
 template <typename Src, int RC>
-__global__ void blur_kernel(Src src, int H, int W, const BlurKernel k, float* __restrict__ out,
+__global__ void blur_kernel(Src src, int H, int W, const BlurKernel k, float* out,
                             unsigned int* maxout) {
     extern __shared__ float sm[];
     dependent_wait();
@@ -491,8 +491,8 @@ constexpr int kNormThreads = 256;  // the launch width; the loops stride by it
 
 // RC > 0 fixes the radius at compile time; RC = 0 takes it from r_arg.
 template <int RC>
-__global__ void normalize_kernel(const float* __restrict__ src, int H, int W, int r_arg, float eps,
-                                 const unsigned int* maxbits, float* __restrict__ out) {
+__global__ void normalize_kernel(const float* src, int H, int W, int r_arg, float eps,
+                                 const unsigned int* maxbits, float* out) {
     extern __shared__ long long smq[];
     dependent_wait();
     let_dependents_start();
