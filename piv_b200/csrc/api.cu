@@ -10,6 +10,7 @@
 #include <cstring>
 #include <deque>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -158,6 +159,68 @@ void count_analyzer(int dev, int by) {
     if (k.analyzers == 0) drop_kept(k);
 }
 
+// The numbered calls of one analyzer that queued work, and what is known of their completion. Frames and
+// the workspace note the calls that used them, and their blocks are handed on only when those calls are
+// known to have completed; all others are freed with cudaFree, as CUDA orders that by itself. Nothing
+// here waits for the whole device: that would break any stream capture in progress on it, and the
+// library's own captures and a caller's relaxed ones allow frames to come and go meanwhile.
+struct CallLog {
+    std::mutex mu;               // also held while the library captures on the analyzer's own stream
+    cudaStream_t own = nullptr;  // the analyzer's own stream, while it lives
+    bool on_own = true;          // calls run on it (false: on a caller's stream, which may be gone at any time)
+    uint64_t calls = 0;
+    uint64_t done = 0;                   // calls up to this one have completed, except the lost ones:
+    uint64_t lost_from = 0, lost_to = 0;  // calls in (from, to] may run later than any wait made here
+    cudaEvent_t mark = nullptr;  // recorded on the caller's stream after call `marked`
+    uint64_t marked = 0;
+
+    ~CallLog() {
+        if (mark) cudaEventDestroy(mark);
+    }
+    // The members below need `mu`.
+    bool lost(uint64_t c) const { return c > lost_from && c <= lost_to; }
+    bool completed(uint64_t c) const { return c <= done && !lost(c); }
+    void lose_pending() {
+        if (done >= calls) return;
+        lost_from = lost_to ? std::min(lost_from, done) : done;
+        lost_to = calls;
+    }
+};
+
+// Waits for call `c` of `log` without waiting for the device; false when its completion cannot be known.
+bool wait_call(CallLog& log, uint64_t c) {
+    std::unique_lock<std::mutex> lk(log.mu);
+    if (log.completed(c)) return true;
+    if (log.lost(c)) return false;
+    uint64_t n = 0;
+    cudaError_t e = cudaErrorUnknown;
+    if (log.on_own && log.own) {
+        cudaEvent_t ev = nullptr;
+        if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess) {
+            e = cudaEventRecord(ev, log.own);
+            n = log.calls;
+            lk.unlock();
+            if (e == cudaSuccess) e = cudaEventSynchronize(ev);
+            cudaEventDestroy(ev);
+            lk.lock();
+        }
+    } else if (!log.on_own && log.marked >= c) {
+        const cudaEvent_t ev = log.mark;
+        n = log.marked;
+        lk.unlock();
+        e = cudaEventSynchronize(ev);
+        lk.lock();
+    } else {
+        return false;
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    log.done = std::max(log.done, n);
+    return log.completed(c);
+}
+
 struct PassBuf {
     PivGridC grid;
     int64_t cells;
@@ -206,7 +269,9 @@ struct PivAnalyzer {
     std::vector<std::vector<PassBuf>> pairs;  // [pair][pass]
     void* arena = nullptr;
     size_t arena_bytes = 0;
+    uint64_t arena_born = 0, arena_call = 0;  // calls made before the arena was, and the last that used it
     unsigned long long* d_counts = nullptr;
+    std::shared_ptr<CallLog> log;  // of analyzers made by piv_analyzer_create
     long long launches = 0;
     // stage timing: per pass, pending (start, end) event pairs and the events to reuse
     bool profiling = false;
@@ -251,6 +316,15 @@ struct PivFrame {
     void* d_raw = nullptr;
     size_t d_raw_bytes = 0;
     float* d_bg = nullptr;
+    // the analyzers whose calls used the frame, with the last such call of each; untracked: some use of
+    // it is known to no log (its image's address was asked for, or a call was lost)
+    struct Use {
+        std::shared_ptr<CallLog> log;
+        uint64_t call;
+    };
+    mutable std::mutex use_mu;
+    mutable std::vector<Use> uses;
+    mutable bool untracked = false;
 };
 
 namespace {
@@ -320,14 +394,125 @@ int use_device(PivAnalyzer* an) {
     return PIV_OK;
 }
 
+void note_use(const PivFrame* f, const std::shared_ptr<CallLog>& log, uint64_t call) {
+    std::lock_guard<std::mutex> lk(f->use_mu);
+    for (PivFrame::Use& u : f->uses)
+        if (u.log == log) {
+            std::lock_guard<std::mutex> ll(log->mu);
+            if (log->lost(u.call)) f->untracked = true;
+            u.call = call;
+            return;
+        }
+    f->uses.erase(std::remove_if(f->uses.begin(), f->uses.end(),
+                                 [](const PivFrame::Use& u) {  // analyzers that are gone
+                                     std::lock_guard<std::mutex> ll(u.log->mu);
+                                     return !u.log->own && u.log->completed(u.call);
+                                 }),
+                  f->uses.end());
+    f->uses.push_back({log, call});
+}
+
+// Counts a call that is about to queue work on the analyzer's stream, using the given frames.
+uint64_t begin_call(PivAnalyzer* an, std::initializer_list<const PivFrame*> frames) {
+    if (!an->log) return 0;
+    uint64_t call = 0;
+    {
+        std::lock_guard<std::mutex> lk(an->log->mu);
+        call = ++an->log->calls;
+        if (!an->log->on_own) {  // a caller's capture: its graph may run at any later time
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(an->cur, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+                an->log->lose_pending();
+        }
+    }
+    for (const PivFrame* f : frames)
+        if (f) note_use(f, an->log, call);
+    return call;
+}
+
+// After the work of an asynchronous analysis has been queued: on a caller's stream, which cannot be
+// waited for later, an event stands for it. (Preparations go without one: an analysis follows.)
+void mark_call(PivAnalyzer* an) {
+    if (!an->log) return;
+    CallLog& log = *an->log;
+    std::lock_guard<std::mutex> lk(log.mu);
+    if (log.on_own || log.lost(log.calls)) return;
+    if (!log.mark && cudaEventCreateWithFlags(&log.mark, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        log.mark = nullptr;
+        return;
+    }
+    if (cudaEventRecord(log.mark, an->cur) == cudaSuccess)
+        log.marked = log.calls;
+    else
+        cudaGetLastError();
+}
+
+// After the analyzer's stream has been waited for: calls up to `call` have completed.
+void calls_completed(PivAnalyzer* an, uint64_t call) {
+    if (!an->log) return;
+    std::lock_guard<std::mutex> lk(an->log->mu);
+    an->log->done = std::max(an->log->done, call);
+}
+
+// Waits for the analyzer's stream.
+cudaError_t wait_stream(PivAnalyzer* an) {
+    const cudaError_t e = cudaStreamSynchronize(an->cur);
+    if (e == cudaSuccess && an->log) calls_completed(an, an->log->calls);
+    return e;
+}
+
+bool frame_idle(const PivFrame* f) {
+    std::vector<PivFrame::Use> uses;
+    {
+        std::lock_guard<std::mutex> lk(f->use_mu);
+        if (f->untracked) return false;
+        uses = f->uses;
+    }
+    for (const PivFrame::Use& u : uses)
+        if (!wait_call(*u.log, u.call)) return false;
+    return true;
+}
+
+bool arena_idle(const PivAnalyzer* an) {
+    if (!an->log || !wait_call(*an->log, an->arena_call)) return false;
+    std::lock_guard<std::mutex> lk(an->log->mu);
+    return an->log->lost_to <= an->arena_born;
+}
+
+// Hands a block on when nothing uses it any more, and frees it otherwise.
+void release_block(int dev, void* p, size_t bytes, bool idle) {
+    if (idle)
+        give_block(dev, p, bytes);
+    else
+        cudaFree(p);
+}
+
+void release_frame(PivFrame* f, bool idle) {  // on the frame's device
+    const size_t n = sizeof(float) * (size_t)f->H * (size_t)f->W;
+    const size_t table = sizeof(long long) * (size_t)(f->H + 1) * (size_t)(f->W + 1);
+    release_block(f->device, f->image, frame_block_bytes(f), idle);
+    release_block(f->device, f->base_store, n, idle);
+    release_block(f->device, f->tmp, n, idle);
+    release_block(f->device, f->sum, table, idle);
+    release_block(f->device, f->sumsq, table, idle);
+    release_block(f->device, f->d_raw, f->d_raw_bytes, idle);
+    release_block(f->device, f->d_bg, n, idle);
+    delete f;
+}
+
 // Per-pair workspace for up to K pairs of (H, W) frames: for every pass, origins, signal status,
 // raw field and the validated field; 8 summary counters per pair.
 int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
-    if (an->arena && an->H == H && an->W == W && an->K >= K) return PIV_OK;
+    const uint64_t call = an->log ? an->log->calls : 0;  // the call in progress
+    if (an->arena && an->H == H && an->W == W && an->K >= K) {
+        an->arena_call = call;
+        return PIV_OK;
+    }
     if (an->arena) {
         CUDA_TRY(cudaStreamSynchronize(an->cur));
-        CUDA_TRY(cudaDeviceSynchronize());  // earlier calls may have run on other streams
-        give_block(an->device, an->arena, an->arena_bytes);
+        if (an->log) calls_completed(an, call - 1);
+        release_block(an->device, an->arena, an->arena_bytes, arena_idle(an));
         an->arena = nullptr;
     }
     an->pairs.clear();
@@ -348,6 +533,8 @@ int ensure_workspace(PivAnalyzer* an, int64_t H, int64_t W, int K) {
     const size_t total = align256(sizeof(unsigned long long) * 8 * (size_t)K) + per_pair * (size_t)K;
     CUDA_TRY(take_block(&an->arena, total));
     an->arena_bytes = total;
+    an->arena_call = call;
+    an->arena_born = call ? call - 1 : 0;
     ++an->epoch;  // the block may have the old one's address, but the layout depends on K, H and W
     char* p = (char*)an->arena;
     auto take = [&](size_t bytes) {
@@ -532,6 +719,11 @@ int run_passes_eager(PivAnalyzer* an, const PivFrame* const* a, const PivFrame* 
 // contents, so new samples in the same frames need no new capture. Tuning, profiling and a
 // stream that the caller is capturing run eagerly.
 int run_passes(PivAnalyzer* an, const PivFrame* const* a, const PivFrame* const* b, int K, bool tune = false) {
+    const uint64_t call = begin_call(an, {});
+    if (an->log)
+        for (int k = 0; k < K; ++k)
+            for (const PivFrame* f : {a[k], b[k]})
+                if (f) note_use(f, an->log, call);
     if (tune || an->profiling || K <= 0) {
         an->pending_key.clear();
         return run_passes_eager(an, a, b, K, tune);
@@ -564,11 +756,14 @@ int run_passes(PivAnalyzer* an, const PivFrame* const* a, const PivFrame* const*
         return run_passes_eager(an, a, b, K, tune);
     }
     // second call with the same key: capture, then replay
+    std::unique_lock<std::mutex> capturing;  // no other thread may wait for the stream meanwhile
+    if (an->log) capturing = std::unique_lock<std::mutex>(an->log->mu);
     CUDA_TRY(cudaStreamBeginCapture(an->cur, cudaStreamCaptureModeRelaxed));
     const long long l0 = an->launches;
     st = run_passes_eager(an, a, b, K, tune);
     cudaGraph_t graph = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(an->cur, &graph);
+    if (capturing) capturing.unlock();
     const long long nl = an->launches - l0;
     an->launches = l0;
     if (st) {
@@ -604,7 +799,7 @@ int copy_summary(PivAnalyzer* an, PivSummaryC* s) {
     if (!s) return PIV_OK;
     unsigned long long c[5];
     CUDA_TRY(cudaMemcpyAsync(c, an->d_counts, sizeof(c), cudaMemcpyDeviceToHost, an->cur));
-    CUDA_TRY(cudaStreamSynchronize(an->cur));
+    CUDA_TRY(wait_stream(an));
     s->no_signal = (int64_t)c[0];
     s->low_ppr = (int64_t)c[1];
     s->median_outliers = (int64_t)c[2];
@@ -701,15 +896,42 @@ int prepare_frames(PivAnalyzer* an, PivFrame* const* frames, const void* const* 
 
 int stage_raw(PivFrame* f, size_t bytes) {
     if (f->d_raw_bytes >= bytes) return PIV_OK;
-    if (f->d_raw) {
-        CUDA_TRY(cudaDeviceSynchronize());
-        give_block(f->device, f->d_raw, f->d_raw_bytes);
-    }
+    if (f->d_raw) release_block(f->device, f->d_raw, f->d_raw_bytes, frame_idle(f));
     f->d_raw = nullptr;
     f->d_raw_bytes = 0;
     CUDA_TRY(take_block(&f->d_raw, bytes));
     f->d_raw_bytes = bytes;
     return PIV_OK;
+}
+
+// Frames may outlive their analyzer: its log stays, closed. `idle`: nothing uses the workspace any more.
+void destroy_analyzer(PivAnalyzer* an, bool idle) {
+    if (!an) return;
+    // Only the analyzer's own stream is known to be alive here.
+    if (an->own) cudaStreamSynchronize(an->own);
+    bool all_idle = idle;
+    if (an->log) {
+        CallLog& log = *an->log;
+        wait_call(log, log.calls);
+        std::lock_guard<std::mutex> lk(log.mu);
+        log.lose_pending();
+        log.own = nullptr;
+        all_idle = log.lost_to == 0;
+    }
+    for (auto& v : an->pending)
+        for (auto& pr : v) {
+            cudaEventDestroy(pr.first);
+            cudaEventDestroy(pr.second);
+        }
+    for (cudaEvent_t e : an->spare) cudaEventDestroy(e);
+    if (an->gexec) {
+        if (!all_idle) cudaDeviceSynchronize();  // a replay may still run on a caller's stream
+        cudaGraphExecDestroy(an->gexec);
+    }
+    release_block(an->device, an->arena, an->arena_bytes, idle);
+    if (an->own) cudaStreamDestroy(an->own);
+    if (an->counted) count_analyzer(an->device, -1);
+    delete an;
 }
 
 __global__ void background_kernel(const void* frames, int dtype, long long count, long long npix, int mode, float* out) {
@@ -779,6 +1001,8 @@ int32_t piv_analyzer_create(const PivConfigC* cfg, PivAnalyzer** out) {
         return fail(PIV_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
     }
     an->cur = an->own;
+    an->log = std::make_shared<CallLog>();
+    an->log->own = an->own;
     an->counted = true;
     count_analyzer(dev, 1);
     *out = an;
@@ -788,27 +1012,7 @@ int32_t piv_analyzer_create(const PivConfigC* cfg, PivAnalyzer** out) {
 void piv_analyzer_destroy(PivAnalyzer* an) {
     if (!an) return;
     cudaSetDevice(an->device);
-    // Only the analyzer's own stream is known to be alive here; cudaFree waits for the device.
-    if (an->own) cudaStreamSynchronize(an->own);
-    for (auto& v : an->pending)
-        for (auto& pr : v) {
-            cudaEventDestroy(pr.first);
-            cudaEventDestroy(pr.second);
-        }
-    for (cudaEvent_t e : an->spare) cudaEventDestroy(e);
-    if (an->gexec) {
-        cudaDeviceSynchronize();  // a replay may still run on a caller's stream
-        cudaGraphExecDestroy(an->gexec);
-    }
-    if (an->arena) {
-        if (cudaDeviceSynchronize() == cudaSuccess)
-            give_block(an->device, an->arena, an->arena_bytes);
-        else
-            cudaFree(an->arena);
-    }
-    if (an->own) cudaStreamDestroy(an->own);
-    if (an->counted) count_analyzer(an->device, -1);
-    delete an;
+    destroy_analyzer(an, arena_idle(an));
 }
 
 int32_t piv_num_passes(const PivAnalyzer* an) {
@@ -830,7 +1034,13 @@ int32_t piv_pass_grid(const PivAnalyzer* an, int64_t height, int64_t width, int3
 
 int32_t piv_analyzer_set_stream(PivAnalyzer* an, void* stream) {
     if (!an) return fail(PIV_ERR_ARGUMENT, "null analyzer");
-    an->cur = stream ? (cudaStream_t)stream : an->own;
+    const cudaStream_t next = stream ? (cudaStream_t)stream : an->own;
+    if (an->log && next != an->cur) {
+        std::lock_guard<std::mutex> lk(an->log->mu);
+        an->log->lose_pending();  // the old stream may be gone before anyone waits for it
+        an->log->on_own = next == an->own;
+    }
+    an->cur = next;
     return PIV_OK;
 }
 
@@ -838,7 +1048,7 @@ int32_t piv_analyzer_sync(PivAnalyzer* an) {
     if (!an) return fail(PIV_ERR_ARGUMENT, "null analyzer");
     int st = use_device(an);
     if (st) return st;
-    CUDA_TRY(cudaStreamSynchronize(an->cur));
+    CUDA_TRY(wait_stream(an));
     return check_device_error(an->device);
 }
 
@@ -848,7 +1058,7 @@ int32_t piv_analyzer_autotune(PivAnalyzer* an, const PivFrame* a, const PivFrame
     if (!an) return fail(PIV_ERR_ARGUMENT, "null analyzer");
     int st = run_passes(an, a, b, true);
     if (st) return st;
-    CUDA_TRY(cudaStreamSynchronize(an->cur));
+    CUDA_TRY(wait_stream(an));
     return PIV_OK;
 }
 
@@ -891,7 +1101,7 @@ int32_t piv_analyzer_profile(PivAnalyzer* an, int32_t pass, double* correlate_ms
     double ms = 0.0;
     int64_t n = 0;
     if (pass >= 0 && pass < (int32_t)an->pending.size()) {
-        CUDA_TRY(cudaStreamSynchronize(an->cur));
+        CUDA_TRY(wait_stream(an));
         for (auto& pr : an->pending[pass]) {
             float t = 0.0f;
             CUDA_TRY(cudaEventElapsedTime(&t, pr.first, pr.second));
@@ -933,26 +1143,9 @@ int32_t piv_frame_create(PivAnalyzer* an, int64_t height, int64_t width, PivFram
 
 void piv_frame_destroy(PivFrame* f) {
     if (!f) return;
-    // A frame may outlive its analyzer: touch nothing of it. Work that reads the frame may be queued on
-    // any stream, so its blocks are handed on only when the device is idle.
+    // A frame may outlive its analyzer: touch nothing of it but its log.
     cudaSetDevice(f->device);
-    if (cudaDeviceSynchronize() == cudaSuccess) {
-        const size_t n = sizeof(float) * (size_t)f->H * (size_t)f->W;
-        const size_t table = sizeof(long long) * (size_t)(f->H + 1) * (size_t)(f->W + 1);
-        give_block(f->device, f->image, frame_block_bytes(f));
-        give_block(f->device, f->base_store, n);
-        give_block(f->device, f->tmp, n);
-        give_block(f->device, f->sum, table);
-        give_block(f->device, f->sumsq, table);
-        give_block(f->device, f->d_raw, f->d_raw_bytes);
-        give_block(f->device, f->d_bg, n);
-    } else {  // a failed device, or a capture in progress: nothing of this frame is handed on
-        cudaGetLastError();
-        for (void* p : {(void*)f->image, (void*)f->base_store, (void*)f->tmp, (void*)f->sum, (void*)f->sumsq, f->d_raw,
-                        (void*)f->d_bg})
-            cudaFree(p);
-    }
-    delete f;
+    release_frame(f, frame_idle(f));
 }
 
 int32_t piv_frame_prepare_device(PivAnalyzer* an, PivFrame* f, const void* raw_dev, int32_t dtype,
@@ -961,6 +1154,7 @@ int32_t piv_frame_prepare_device(PivAnalyzer* an, PivFrame* f, const void* raw_d
     if (!dtype_size(dtype)) return fail(PIV_ERR_ARGUMENT, "unknown dtype %d", dtype);
     int st = use_device(an);
     if (st) return st;
+    begin_call(an, {f});
     return prepare_common(an, f, raw_dev, dtype, pre, background_dev);
 }
 
@@ -974,6 +1168,7 @@ int32_t piv_frame_prepare(PivAnalyzer* an, PivFrame* f, const void* raw, int32_t
     const size_t n = (size_t)f->H * (size_t)f->W;
     st = stage_raw(f, es * n);
     if (st) return st;
+    begin_call(an, {f});
     CUDA_TRY(cudaMemcpyAsync(f->d_raw, raw, es * n, cudaMemcpyHostToDevice, an->cur));
     const float* bg = nullptr;
     if (background) {
@@ -988,6 +1183,7 @@ int32_t piv_frame_set_prepared(PivAnalyzer* an, PivFrame* f, const float* image,
     if (!an || !f || !image) return fail(PIV_ERR_ARGUMENT, "null argument");
     int st = use_device(an);
     if (st) return st;
+    begin_call(an, {f});
     const size_t n = (size_t)f->H * (size_t)f->W;
     CUDA_TRY(cudaMemcpyAsync(f->image, image, sizeof(float) * n, cudaMemcpyHostToDevice, an->cur));
     f->nonneg = false;  // unknown: statistics are always built
@@ -1005,7 +1201,7 @@ int32_t piv_frame_set_prepared(PivAnalyzer* an, PivFrame* f, const float* image,
     an->launches += nl;
     f->stats_valid = true;
     f->strips = true;
-    CUDA_TRY(cudaStreamSynchronize(an->cur));
+    CUDA_TRY(wait_stream(an));
     return PIV_OK;
 }
 
@@ -1015,6 +1211,7 @@ int32_t piv_frame_set_prepared_tables(PivAnalyzer* an, PivFrame* f, const float*
     if (!f->words) return fail(PIV_ERR_ARGUMENT, "frame has no scratch");
     int st = use_device(an);
     if (st) return st;
+    begin_call(an, {f});
     const size_t n = (size_t)f->H * (size_t)f->W;
     const size_t cells = (size_t)(f->H + 1) * (size_t)(f->W + 1);
     CUDA_TRY(cudaMemcpyAsync(f->image, image, sizeof(float) * n, cudaMemcpyHostToDevice, an->cur));
@@ -1034,7 +1231,7 @@ int32_t piv_frame_set_prepared_tables(PivAnalyzer* an, PivFrame* f, const float*
     an->launches += nl;
     unsigned int bad = 0;
     CUDA_TRY(cudaMemcpyAsync(&bad, nonfinite, sizeof(bad), cudaMemcpyDeviceToHost, an->cur));
-    CUDA_TRY(cudaStreamSynchronize(an->cur));
+    CUDA_TRY(wait_stream(an));
     f->base = f->image;  // the tables stand for the base image, which is not needed itself
     if (bad) {
         f->stats_valid = false;
@@ -1048,12 +1245,18 @@ int32_t piv_frame_download(PivAnalyzer* an, const PivFrame* f, float* image) {
     if (!an || !f || !image) return fail(PIV_ERR_ARGUMENT, "null argument");
     int st = use_device(an);
     if (st) return st;
+    begin_call(an, {f});
     CUDA_TRY(cudaMemcpyAsync(image, f->image, sizeof(float) * f->H * f->W, cudaMemcpyDeviceToHost, an->cur));
-    CUDA_TRY(cudaStreamSynchronize(an->cur));
+    CUDA_TRY(wait_stream(an));
     return PIV_OK;
 }
 
-const float* piv_frame_image_device(const PivFrame* f) { return f ? f->image : nullptr; }
+const float* piv_frame_image_device(const PivFrame* f) {
+    if (!f) return nullptr;
+    std::lock_guard<std::mutex> lk(f->use_mu);
+    f->untracked = true;  // the caller's own work may read it
+    return f->image;
+}
 
 int32_t piv_background_device(PivAnalyzer* an, const void* frames_dev, int32_t dtype, int64_t count, int64_t height,
                               int64_t width, int32_t mode, float* out_dev) {
@@ -1127,7 +1330,9 @@ int32_t piv_analyze_device(PivAnalyzer* an, const PivFrame* a, const PivFrame* b
     if (!an) return fail(PIV_ERR_ARGUMENT, "null analyzer");
     int st = run_passes(an, a, b);
     if (st) return st;
-    return export_fields(an, 1, dx, dy, peak_ratio, flags, (unsigned long long*)summary_dev, 5);
+    st = export_fields(an, 1, dx, dy, peak_ratio, flags, (unsigned long long*)summary_dev, 5);
+    mark_call(an);
+    return st;
 }
 
 int32_t piv_analyze(PivAnalyzer* an, const PivFrame* a, const PivFrame* b, float* dx, float* dy, float* peak_ratio,
@@ -1143,7 +1348,7 @@ int32_t piv_analyze(PivAnalyzer* an, const PivFrame* a, const PivFrame* b, float
     if (flags) CUDA_TRY(cudaMemcpyAsync(flags, last.flags, c, cudaMemcpyDeviceToHost, an->cur));
     st = copy_summary(an, summary);
     if (st) return st;
-    CUDA_TRY(cudaStreamSynchronize(an->cur));
+    CUDA_TRY(wait_stream(an));
     return check_device_error(an->device);
 }
 
@@ -1171,7 +1376,7 @@ int32_t piv_analyze_traced(PivAnalyzer* an, const PivFrame* a, const PivFrame* b
     }
     st = copy_summary(an, summary);
     if (st) return st;
-    CUDA_TRY(cudaStreamSynchronize(an->cur));
+    CUDA_TRY(wait_stream(an));
     return PIV_OK;
 }
 
@@ -1222,7 +1427,7 @@ int place_windows(PivAnalyzer* an, int64_t height, int64_t width, const PivGridC
     an->launches += 1;
     if (e == cudaSuccess) e = cudaMemcpyAsync(origins, d_org, 16 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && corners) e = cudaMemcpyAsync(corners, d_corners, 32 * c, cudaMemcpyDeviceToHost, an->cur);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(an->cur);
+    if (e == cudaSuccess) e = wait_stream(an);
     if (e == cudaSuccess)
         give_block(an->device, buf, buf_bytes);  // the stream has been waited for
     else
@@ -1263,6 +1468,7 @@ int32_t piv_correlate_origins(PivAnalyzer* an, const PivFrame* a, const PivFrame
     if (st) return st;
     const bool use_stats = needs_stats(an, a) || needs_stats(an, b);
     if (use_stats && !(a->stats_valid && b->stats_valid)) return fail(PIV_ERR_ARGUMENT, "frame statistics missing");
+    begin_call(an, {a, b});
     const size_t c = (size_t)ncells;
     void* buf = nullptr;
     const size_t buf_bytes = align256(16 * c) + align256(c) + 3 * align256(4 * c) + align256(c) + 256;
@@ -1303,7 +1509,7 @@ int32_t piv_correlate_origins(PivAnalyzer* an, const PivFrame* a, const PivFrame
     if (e == cudaSuccess && dy) e = cudaMemcpyAsync(dy, d_dy, 4 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && peak_ratio) e = cudaMemcpyAsync(peak_ratio, d_ppr, 4 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && flags) e = cudaMemcpyAsync(flags, d_fl, c, cudaMemcpyDeviceToHost, an->cur);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(an->cur);
+    if (e == cudaSuccess) e = wait_stream(an);
     if (e == cudaSuccess)
         give_block(an->device, buf, buf_bytes);  // the stream has been waited for
     else
@@ -1336,6 +1542,7 @@ int32_t piv_correlate_deform(PivAnalyzer* an, const PivFrame* a, const PivFrame*
     if (st) return st;
     const bool use_stats = needs_stats(an, a) || needs_stats(an, b);
     if (use_stats && !(a->stats_valid && b->stats_valid)) return fail(PIV_ERR_ARGUMENT, "frame statistics missing");
+    begin_call(an, {a, b});
     const size_t c = (size_t)ncells;
     void* buf = nullptr;
     const size_t buf_bytes = align256(16 * c) + align256(32 * c) + align256(c) + 3 * align256(4 * c) + align256(c) + 256;
@@ -1377,7 +1584,7 @@ int32_t piv_correlate_deform(PivAnalyzer* an, const PivFrame* a, const PivFrame*
     if (e == cudaSuccess && dy) e = cudaMemcpyAsync(dy, d_dy, 4 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && peak_ratio) e = cudaMemcpyAsync(peak_ratio, d_ppr, 4 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && flags) e = cudaMemcpyAsync(flags, d_fl, c, cudaMemcpyDeviceToHost, an->cur);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(an->cur);
+    if (e == cudaSuccess) e = wait_stream(an);
     if (e == cudaSuccess)
         give_block(an->device, buf, buf_bytes);  // the stream has been waited for
     else
@@ -1510,7 +1717,7 @@ int32_t piv_validate_field(PivAnalyzer* an, int64_t ny, int64_t nx, const float*
     if (e == cudaSuccess && out_dy) e = cudaMemcpyAsync(out_dy, o_dy, 4 * c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess && out_flags) e = cudaMemcpyAsync(out_flags, fo, c, cudaMemcpyDeviceToHost, an->cur);
     if (e == cudaSuccess) e = cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, an->cur);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(an->cur);
+    if (e == cudaSuccess) e = wait_stream(an);
     if (e == cudaSuccess)
         give_block(an->device, buf, buf_bytes);  // the stream has been waited for
     else
@@ -1531,7 +1738,9 @@ int32_t piv_analyze_batch_device(PivAnalyzer* an, const PivFrame* const* a, cons
     if (!an || !a || !b) return fail(PIV_ERR_ARGUMENT, "null argument");
     int st = run_passes(an, a, b, count);
     if (st) return st;
-    return export_fields(an, count, dx, dy, peak_ratio, flags, (unsigned long long*)summaries_dev, 8);
+    st = export_fields(an, count, dx, dy, peak_ratio, flags, (unsigned long long*)summaries_dev, 8);
+    mark_call(an);
+    return st;
 }
 
 namespace {
@@ -1642,11 +1851,12 @@ int32_t piv_batch_create(const PivAnalyzer* parent, int64_t height, int64_t widt
 
 void piv_batch_destroy(PivBatch* bt) {
     if (!bt) return;
+    bool idle = false;
     if (bt->an) {
         cudaSetDevice(bt->an->device);
         // The batch's kernels may run on a stream it borrowed (piv_batch_set_stream), which may
         // already be gone; waiting for the device needs no stream handle.
-        cudaDeviceSynchronize();
+        idle = cudaDeviceSynchronize() == cudaSuccess;
         bt->an->cur = bt->an->own;
     }
     for (cudaStream_t st : {bt->up, bt->down})
@@ -1659,10 +1869,10 @@ void piv_batch_destroy(PivBatch* bt) {
     for (cudaEvent_t ev : {bt->uploaded, bt->computed, bt->hdone})
         if (ev) cudaEventDestroy(ev);
     if (bt->hsums) cudaFreeHost(bt->hsums);
-    for (PivFrame* f : bt->frames) piv_frame_destroy(f);
+    for (PivFrame* f : bt->frames) release_frame(f, idle);
     cudaFree(bt->raw);
     cudaFree(bt->out);
-    piv_analyzer_destroy(bt->an);
+    destroy_analyzer(bt->an, idle);
     delete bt;
 }
 
@@ -1769,15 +1979,16 @@ int32_t piv_pipeline_create(const PivAnalyzer* parent, int64_t height, int64_t w
 void piv_pipeline_destroy(PivPipeline* pl) {
     if (!pl) return;
     cudaSetDevice(pl->device);
+    bool idle = true;
     for (cudaStream_t st : {pl->up, pl->prep, pl->comp, pl->down})
-        if (st) cudaStreamSynchronize(st);
+        if (st) idle &= cudaStreamSynchronize(st) == cudaSuccess;
     for (auto& s : pl->slots) {
-        if (s.fa) piv_frame_destroy(s.fa);
-        if (s.fb) piv_frame_destroy(s.fb);
+        if (s.fa) release_frame(s.fa, idle);
+        if (s.fb) release_frame(s.fb, idle);
         for (cudaEvent_t ev : {s.uploaded, s.prepared, s.computed, s.done})
             if (ev) cudaEventDestroy(ev);
         if (s.sums) cudaFreeHost(s.sums);
-        piv_analyzer_destroy(s.an);
+        destroy_analyzer(s.an, idle);
     }
     for (cudaStream_t st : {pl->up, pl->prep, pl->comp, pl->down})
         if (st) cudaStreamDestroy(st);
