@@ -74,19 +74,21 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Device blocks of destroyed frames, of analyzers' workspaces and of the blocking stage calls, kept for
 // the next ones: a program that makes frames for every pair spent more time in cudaMalloc and cudaFree
-// than in the analysis (1024 x 768 pair, host to host: 1.55 ms and more, 0.30 ms with the blocks kept;
+// than in the analysis (1024 x 768 pair, host to host: 1.55 ms and more, 0.27 ms with the blocks kept;
 // the first pass of a new analyzer on a 1024 x 1024 pair 0.70 -> 0.26 ms). A block comes here only when
-// no work can be using it (its giver has waited for the device or for its stream). At most kKeptBytes
-// are kept per device, in no one's name; they go back to the device when an allocation fails and when
-// the device's last analyzer is destroyed.
+// no work can be using it. At most kKeptBytes are kept per device, in no one's name: the oldest blocks
+// make room for new ones, and all go back to the device when an allocation fails and when the device's
+// last analyzer is destroyed. 256 MiB hold the two frames of a default-conditioned 9 Mpixel pair (14
+// bytes per 16-bit pixel), or of a masked 4 Mpixel pair (30); it is memory that others cannot have.
 constexpr size_t kKeptBytes = (size_t)256 << 20;
 struct KeptBlocks {
-    std::multimap<size_t, void*> free;
+    std::vector<std::pair<size_t, void*>> free;  // (size, block), oldest first
     size_t bytes = 0;
     int analyzers = 0;  // live analyzers on the device
 };
-std::mutex g_kept_mu;
-std::map<int, KeptBlocks> g_kept;
+// Never destroyed: a program's own objects may be given back while the process exits.
+std::mutex& g_kept_mu = *new std::mutex();
+std::map<int, KeptBlocks>& g_kept = *new std::map<int, KeptBlocks>();
 
 void drop_kept(KeptBlocks& k) {  // with g_kept_mu held and the device current
     for (auto& b : k.free) cudaFree(b.second);
@@ -122,13 +124,13 @@ cudaError_t take_block(T** out, size_t bytes) {
     {
         std::lock_guard<std::mutex> lk(g_kept_mu);
         KeptBlocks& k = g_kept[dev];
-        auto it = k.free.find(want);
-        if (it != k.free.end()) {
-            *out = static_cast<T*>(it->second);
-            k.free.erase(it);
-            k.bytes -= want;
-            return cudaSuccess;
-        }
+        for (size_t i = k.free.size(); i-- > 0;)
+            if (k.free[i].first == want) {
+                *out = static_cast<T*>(k.free[i].second);
+                k.free.erase(k.free.begin() + (ptrdiff_t)i);
+                k.bytes -= want;
+                return cudaSuccess;
+            }
     }
     void* p = nullptr;
     e = device_malloc(&p, want);
@@ -140,16 +142,23 @@ cudaError_t take_block(T** out, size_t bytes) {
 void give_block(int dev, void* p, size_t bytes) {
     if (!p) return;
     const size_t size = block_bytes(bytes);
+    std::vector<void*> out = {p};  // what is freed below: the block itself, or the oldest ones it displaces
     {
         std::lock_guard<std::mutex> lk(g_kept_mu);
         KeptBlocks& k = g_kept[dev];
-        if (k.analyzers > 0 && k.bytes + size <= kKeptBytes) {
-            k.free.emplace(size, p);
+        if (k.analyzers > 0 && size <= kKeptBytes) {
+            out.clear();
+            size_t n = 0;
+            for (; k.bytes + size > kKeptBytes; ++n) {
+                out.push_back(k.free[n].second);
+                k.bytes -= k.free[n].first;
+            }
+            k.free.erase(k.free.begin(), k.free.begin() + (ptrdiff_t)n);
+            k.free.emplace_back(size, p);
             k.bytes += size;
-            return;
         }
     }
-    cudaFree(p);
+    for (void* q : out) cudaFree(q);
 }
 
 void count_analyzer(int dev, int by) {
