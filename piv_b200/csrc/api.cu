@@ -96,20 +96,28 @@ void drop_kept(KeptBlocks& k) {  // with g_kept_mu held and the device current
     k.bytes = 0;
 }
 
-// cudaMalloc on the current device that first gives the kept blocks back when memory runs out.
-cudaError_t device_malloc(void** out, size_t bytes) {
-    cudaError_t e = cudaMalloc(out, bytes);
-    if (e != cudaErrorMemoryAllocation) return e;
+// Gives the current device's kept blocks back to it; false when there were none.
+bool give_back_kept() {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return e;
-    {
-        std::lock_guard<std::mutex> lk(g_kept_mu);
-        auto it = g_kept.find(dev);
-        if (it == g_kept.end() || it->second.free.empty()) return e;
-        drop_kept(it->second);
-    }
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lk(g_kept_mu);
+    auto it = g_kept.find(dev);
+    if (it == g_kept.end() || it->second.free.empty()) return false;
+    drop_kept(it->second);
+    return true;
+}
+
+// Runs an allocation on the current device, and once more without the kept blocks when memory runs out.
+template <class Alloc>
+cudaError_t with_kept_memory(const Alloc& alloc) {
+    const cudaError_t e = alloc();
+    if (e != cudaErrorMemoryAllocation || !give_back_kept()) return e;
     cudaGetLastError();  // not a sticky error
-    return cudaMalloc(out, bytes);
+    return alloc();
+}
+
+cudaError_t device_malloc(void** out, size_t bytes) {
+    return with_kept_memory([&] { return cudaMalloc(out, bytes); });
 }
 
 size_t block_bytes(size_t bytes) { return (bytes + 0xffff) & ~(size_t)0xffff; }  // multiples of 64 KiB
@@ -2364,8 +2372,9 @@ int admit_request(PivServer* sv, Request* r, bool inject_failure) {
     const size_t hw = (size_t)r->H * (size_t)r->W;
     const bool chain = r->pre.smooth_sigma > 0.0f || r->pre.normalize_radius > 0;
     const bool both = r->pre.smooth_sigma > 0.0f && r->pre.normalize_radius > 0;
-    if (inject_failure) return kAdmitOutOfMemory;
-    const cudaError_t ae = cudaMallocFromPoolAsync(&r->mem, r->bytes, sv->pool, sv->up);
+    const cudaError_t ae = with_kept_memory([&] {
+        return inject_failure ? cudaErrorMemoryAllocation : cudaMallocFromPoolAsync(&r->mem, r->bytes, sv->pool, sv->up);
+    });
     if (ae == cudaErrorMemoryAllocation) {
         cudaGetLastError();  // not a sticky error: clear it and report
         r->mem = nullptr;
@@ -2871,7 +2880,7 @@ int32_t piv_server_reserve(PivServer* sv, int64_t bytes, int64_t* reserved_bytes
         for (int64_t left = bytes; left > 0 && e == cudaSuccess;) {
             const int64_t n = std::min(left, kChunk);
             void* p = nullptr;
-            e = cudaMallocFromPoolAsync(&p, (size_t)n, sv->pool, s);
+            e = with_kept_memory([&] { return cudaMallocFromPoolAsync(&p, (size_t)n, sv->pool, s); });
             if (e == cudaSuccess) chunks.push_back(p);
             left -= n;
         }
