@@ -116,9 +116,13 @@ cudaError_t with_kept_memory(const Alloc& alloc) {
     return alloc();
 }
 
-cudaError_t device_malloc(void** out, size_t bytes) {
+}  // namespace
+
+cudaError_t pivb200::device_malloc(void** out, size_t bytes) {
     return with_kept_memory([&] { return cudaMalloc(out, bytes); });
 }
+
+namespace {
 
 size_t block_bytes(size_t bytes) { return (bytes + 0xffff) & ~(size_t)0xffff; }  // multiples of 64 KiB
 

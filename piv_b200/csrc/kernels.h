@@ -11,6 +11,10 @@ namespace pivb200 {
 // Sets the message piv_last_error returns on this host thread.
 void set_last_error(const char* msg);
 
+// cudaMalloc on the current device; when memory runs out, the device blocks kept for later use go back
+// to the device first (api.cu).
+cudaError_t device_malloc(void** out, size_t bytes);
+
 // Launches a kernel that calls dependent_wait() (common.cuh), allowed to start before the previous
 // kernel of the stream has ended: its launch, block scheduling and table set-up then overlap that
 // kernel's tail. A short chain is mostly such gaps (one-pass 512 x 512 pair, 6 kernels: 39.0 -> 34.6 us).

@@ -8,7 +8,6 @@
 // statistics use a fixed-order tree and agree to f32 rounding.
 #include <algorithm>
 #include <cmath>
-#include <condition_variable>
 #include <cstdint>
 #include <cstring>
 #include <map>
@@ -58,19 +57,17 @@ __device__ __forceinline__ bool deriv(const float* d, const float* dxf, const ui
 // One launch per field: every block sums its cells in a fixed order, and the block that finishes
 // last adds the block sums in block order and writes the result to mapped host memory, so a call is
 // one kernel and one stream wait. It is bound by that launch-and-wait latency, not by its 9 bytes
-// per cell. The block sums live in a fixed set of device slots: allocating them per call made the
+// per cell. The block sums live in device slots that are kept: allocating them per call made the
 // stream-ordered pool map and unmap memory at every wait, and one thread added the block sums
 // (64 fields of 118 x 66 smoothed and summed: 30-60 -> 1.7 ms, B200).
 constexpr int kFlowThreads = 256;
 constexpr int kFlowBlocks = 296;  // two per SM; larger fields loop
-constexpr int kFlowSlots = 16;    // calls in flight per device; further callers wait for a slot
-constexpr int kFlowMaxDevices = 16;
+constexpr size_t kFlowKept = 64;  // slots kept per device (12 KB each); calls at the same time have one each
 
 struct FlowSlot {
     FlowPartial part[kFlowBlocks];
     unsigned int done;  // blocks finished; the last one sets it back to 0
 };
-__device__ FlowSlot g_flow[kFlowSlots];
 
 // Sum over the block in a fixed order; the result is valid in thread 0.
 __device__ __forceinline__ FlowPartial flow_block_sum(FlowPartial p) {
@@ -95,8 +92,8 @@ __device__ __forceinline__ FlowPartial flow_block_sum(FlowPartial p) {
 
 __global__ void __launch_bounds__(kFlowThreads) flow_kernel(int ny, int nx, float k, float h,
                                                             const float* __restrict__ dx, const float* __restrict__ dy,
-                                                            const uint8_t* __restrict__ fl, float* vort, int slot,
-                                                            FlowPartial* out) {
+                                                            const uint8_t* __restrict__ fl, float* vort,
+                                                            FlowSlot* slot, FlowPartial* out) {
     FlowPartial t{0.0, 0.0, 0.0, 0, 0};
     const long long cells = (long long)ny * nx;
     for (long long c = (long long)blockIdx.x * kFlowThreads + threadIdx.x; c < cells; c += (long long)gridDim.x * kFlowThreads) {
@@ -118,7 +115,7 @@ __global__ void __launch_bounds__(kFlowThreads) flow_kernel(int ny, int nx, floa
         }
     }
     t = flow_block_sum(t);
-    FlowSlot& s = g_flow[slot];
+    FlowSlot& s = *slot;
     __shared__ bool last;
     if (threadIdx.x == 0) {
         s.part[blockIdx.x] = t;
@@ -144,51 +141,67 @@ __global__ void __launch_bounds__(kFlowThreads) flow_kernel(int ny, int nx, floa
     }
 }
 
-// Slots of flow_kernel per device: a call holds one from its launch to the end of its wait. The
-// mapped host block (one result per slot) is made once per process and shared by all devices.
-static std::mutex g_flow_mu;
-static std::condition_variable g_flow_cv;
-static std::map<int, unsigned int> g_flow_used;  // device -> slots in use
-static FlowPartial* g_flow_host = nullptr;       // kFlowSlots results
+// What one call holds from its launch to the end of its wait: a slot and a mapped host word set for the
+// result. A call takes one that is free or makes one, so no call waits for another.
+struct FlowCall {
+    FlowSlot* slot = nullptr;
+    FlowPartial* host = nullptr;
+    FlowPartial* out = nullptr;  // the device's address of *host
+};
+// Never destroyed: calls may come while the process exits.
+static std::mutex& g_flow_mu = *new std::mutex();
+static std::map<int, std::vector<FlowCall>>& g_flow_free = *new std::map<int, std::vector<FlowCall>>();
+
+static void flow_call_free(const FlowCall& c) {
+    cudaFree(c.slot);
+    cudaFreeHost(c.host);
+}
+
+static cudaError_t flow_call_make(FlowCall* c, cudaStream_t s) {
+    cudaError_t e = device_malloc(reinterpret_cast<void**>(&c->slot), sizeof(FlowSlot));
+    if (e == cudaSuccess)
+        e = cudaHostAlloc(reinterpret_cast<void**>(&c->host), sizeof(FlowPartial), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->out), c->host, 0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(&c->slot->done, 0, sizeof(c->slot->done), s);
+    return e;
+}
 
 cudaError_t flow_stats_device(int ny, int nx, float step, double dt_s, const float* dx, const float* dy,
                               const uint8_t* flags, float* vort, FlowStatsHost* stats, cudaStream_t s) {
-    const int cells = ny * nx;
+    const long long cells = (long long)ny * nx;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    int slot = 0;
+    FlowCall c;
     {
-        std::unique_lock<std::mutex> lk(g_flow_mu);
-        if (!g_flow_host) {
-            void* m = nullptr;
-            e = cudaHostAlloc(&m, sizeof(FlowPartial) * kFlowSlots * kFlowMaxDevices, cudaHostAllocPortable | cudaHostAllocMapped);
-            if (e != cudaSuccess) return e;
-            g_flow_host = static_cast<FlowPartial*>(m);
+        std::lock_guard<std::mutex> lk(g_flow_mu);
+        std::vector<FlowCall>& free = g_flow_free[dev];
+        if (!free.empty()) {
+            c = free.back();
+            free.pop_back();
         }
-        if (dev >= kFlowMaxDevices) return cudaErrorInvalidDevice;
-        unsigned int& used = g_flow_used[dev];
-        g_flow_cv.wait(lk, [&] { return used != (1u << kFlowSlots) - 1; });
-        while (used >> slot & 1u) ++slot;
-        used |= 1u << slot;
     }
-    FlowPartial* host = g_flow_host + dev * kFlowSlots + slot;
-    FlowPartial* out = nullptr;
-    e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&out), host, 0);
+    if (!c.slot) e = flow_call_make(&c, s);
     if (e == cudaSuccess) {
-        const int blocks = std::min((cells + kFlowThreads - 1) / kFlowThreads, kFlowBlocks);
-        flow_kernel<<<blocks, kFlowThreads, 0, s>>>(ny, nx, (float)(1.0 / dt_s), step, dx, dy, flags, vort, slot, out);
+        const int blocks = (int)std::min<long long>((cells + kFlowThreads - 1) / kFlowThreads, kFlowBlocks);
+        flow_kernel<<<blocks, kFlowThreads, 0, s>>>(ny, nx, (float)(1.0 / dt_s), step, dx, dy, flags, vort, c.slot, c.out);
         e = cudaGetLastError();
         const cudaError_t w = cudaStreamSynchronize(s);
         if (e == cudaSuccess) e = w;
     }
-    const FlowPartial t = *host;
+    if (e != cudaSuccess) {  // the slot's count may not be 0
+        flow_call_free(c);
+        return e;
+    }
+    const FlowPartial t = *c.host;
+    bool keep = false;
     {
         std::lock_guard<std::mutex> lk(g_flow_mu);
-        g_flow_used[dev] &= ~(1u << slot);
+        std::vector<FlowCall>& free = g_flow_free[dev];
+        keep = free.size() < kFlowKept;
+        if (keep) free.push_back(c);
     }
-    g_flow_cv.notify_one();
-    if (e != cudaSuccess) return e;
+    if (!keep) flow_call_free(c);
     auto mean = [](double v, long long c) { return c > 0 ? (float)(v / (double)c) : NAN; };
     stats->vorticity_mean = mean(t.ws, t.nw);
     stats->vorticity_abs_mean = mean(t.wa, t.nw);
