@@ -16,6 +16,8 @@
 #include <thread>
 #include <vector>
 
+#include <cuda.h>
+
 #include "../../include/piv_b200.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -1295,17 +1297,46 @@ int32_t piv_background_device(PivAnalyzer* an, const void* frames_dev, int32_t d
 
 namespace {
 
-// Whether a kernel on `dev` can write all of these buffers directly (null ones are skipped). Other
-// memory (another device's, unregistered host memory) keeps the copy commands.
-bool kernel_writable(int dev, std::initializer_list<const void*> ptrs) {
-    for (const void* p : ptrs) {
-        if (!p) continue;
-        cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+struct OutBuffer {
+    const void* p;  // nullable
+    size_t bytes, align;
+};
+
+// Whether a kernel on `dev` can write all of these buffers directly: aligned for its stores, apart from
+// each other, whole within one allocation, and at their own address on the device. Everything else
+// (another device's memory, unregistered host memory, odd addresses, buffers that are too short) is left
+// to the copy commands, which take it or report it.
+bool kernel_writable(int dev, std::initializer_list<OutBuffer> out) {
+    using Query = CUresult (*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found{};
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-            return false;
+            f = nullptr;
         }
-        if (at.type == cudaMemoryTypeUnregistered || (at.type == cudaMemoryTypeDevice && at.device != dev)) return false;
+        return reinterpret_cast<Query>(f);
+    }();
+    if (!query) return false;
+    for (const OutBuffer& b : out) {
+        if (!b.p) continue;
+        const uintptr_t p = (uintptr_t)b.p;
+        if (p % b.align) return false;
+        for (const OutBuffer& o : out)
+            if (&o != &b && o.p && p < (uintptr_t)o.p + o.bytes && (uintptr_t)o.p < p + b.bytes) return false;
+        unsigned int type = 0;
+        int ordinal = -1;
+        CUdeviceptr here = 0, start = 0;
+        size_t size = 0;
+        CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                      CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                      CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+        void* into[] = {&type, &ordinal, &here, &start, &size};
+        if (query(5, what, into, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+        if ((type != CU_MEMORYTYPE_DEVICE && type != CU_MEMORYTYPE_HOST) || (CUdeviceptr)p != here) return false;
+        if (type == CU_MEMORYTYPE_DEVICE && ordinal != dev) return false;
+        if (p < start || b.bytes > size || p - start > size - b.bytes) return false;
     }
     return true;
 }
@@ -1314,8 +1345,10 @@ bool kernel_writable(int dev, std::initializer_list<const void*> ptrs) {
 // buffers on the analyzer's stream; `counts_out` has `count_stride` counters per pair.
 int export_fields(PivAnalyzer* an, int count, float* dx, float* dy, float* peak_ratio, uint8_t* flags,
                   unsigned long long* counts_out, int count_stride) {
-    const size_t c = (size_t)an->pairs[0].back().cells;
-    if (kernel_writable(an->device, {dx, dy, peak_ratio, flags, counts_out})) {
+    const size_t c = (size_t)an->pairs[0].back().cells, n = c * (size_t)count;
+    const size_t count_bytes = sizeof(unsigned long long) * ((size_t)count_stride * (size_t)(count - 1) + 5);
+    if (kernel_writable(an->device, {{dx, 4 * n, 4}, {dy, 4 * n, 4}, {peak_ratio, 4 * n, 4}, {flags, n, 1},
+                                     {counts_out, count_bytes, 8}})) {
         std::vector<ExportItem> items(count);
         for (int k = 0; k < count; ++k) {
             const PassBuf& last = an->pairs[k].back();
