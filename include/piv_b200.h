@@ -142,14 +142,15 @@ int64_t piv_analyzer_launches(const PivAnalyzer* an);
 /* Launch-geometry autotuning (no counterpart in the reference; the batching form of this
  * project): analyses the pair once while timing, for every pass, each launch variant of the
  * correlation kernel of that window size on the live data, and keeps the fastest per window
- * size for this analyzer. Variants of one size differ only in threads per block, register cap
- * and sampler, never in arithmetic: results are bit-identical whichever is chosen. Blocking. */
+ * size for this analyzer. Variants of one size differ only in threads per block and register cap,
+ * never in arithmetic: results are bit-identical whichever is chosen. Blocking. */
 int32_t piv_analyzer_autotune(PivAnalyzer* an, const PivFrame* a, const PivFrame* b);
 /* Launch variants of the FP32 kernel for `window` (uniform windows), and pinning one of them for
- * this analyzer (for tests and external tuning; results are identical whichever is used). */
+ * this analyzer (for tests and external tuning; results are identical whichever is used). Numbers
+ * that earlier builds offered beyond these are accepted and run variant 0. */
 int32_t piv_num_variants(int32_t window);
 int32_t piv_analyzer_set_variant(PivAnalyzer* an, int32_t window, int32_t variant);
-/* Name of the variant in use for `window` ("<n>/T<lanes per line>/G<groups>/B<min blocks>/<sampler>"). */
+/* Name of the variant in use for `window` ("<n>/T<lanes per line>/G<groups>/B<min blocks>", deformed windows with "/deform"). */
 int32_t piv_analyzer_variant(const PivAnalyzer* an, int32_t window, char* name, int32_t capacity);
 /* Stage timing (no counterpart in the reference, which has only wall-clock splits,
  * swift/Sources/PIVKit/Run.swift:189-196): when enabled, CUDA events bracket every correlation

@@ -1103,9 +1103,9 @@ int32_t piv_analyzer_set_variant(PivAnalyzer* an, int32_t window, int32_t v) {
     if (!an) return fail(PIV_ERR_ARGUMENT, "null analyzer");
     if (!corr_supported(window)) return fail(PIV_ERR_UNSUPPORTED, "window size %d", window);
     const int kind = an->deform ? 1 : 0;
-    if (v < 0 || v >= corr_num_variants(window, kind))
+    if (v < 0 || v >= corr_pinnable_variants(window, kind))
         return fail(PIV_ERR_ARGUMENT, "variant %d out of range for window %d", v, window);
-    an->variant[kind][window] = v;
+    an->variant[kind][window] = v < corr_num_variants(window, kind) ? v : 0;
     an->fp32_faster[kind][window] = true;  // an explicit FP32 launch variant
     ++an->epoch;
     return PIV_OK;

@@ -976,6 +976,11 @@ int corr_num_variants(int n, bool deform) {
     return c;
 }
 
+int corr_pinnable_variants(int n, bool deform) {
+    const int kept = deform ? (n == 64 ? 2 : 0) : n == 16 ? 8 : n == 32 ? 6 : n == 8 ? 4 : n == 96 || n == 128 ? 2 : 3;
+    return std::max(corr_num_variants(n, deform), kept);
+}
+
 const char* corr_variant_name(int n, int v, bool deform) {
     int c = 0;
     const CorrVariant* vs = variants(n, deform, &c);

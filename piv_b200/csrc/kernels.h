@@ -80,6 +80,9 @@ cudaError_t corr_init_device();  // uploads the root-of-unity table to the curre
 cudaError_t launch_correlate(int n, const CorrParams& p, cudaStream_t s);
 // Launch variants of one window size (identical results; different geometry), for the autotuner.
 int corr_num_variants(int n, bool deform = false);
+// Numbers a caller may pin: those above, and the ones of launch shapes that there were before (other
+// samplers and caps, with the same results), which now stand for variant 0.
+int corr_pinnable_variants(int n, bool deform);
 const char* corr_variant_name(int n, int v, bool deform = false);
 cudaError_t launch_correlate_variant(int n, int v, const CorrParams& p, cudaStream_t s);
 // All items share window size n and either all have corners (deformed windows) or none; v
