@@ -251,24 +251,26 @@ __device__ int collect_neighbours(const float (*u)[RU], const float (*v)[RU], co
     return c;
 }
 
-// Validation of one 32 x TY tile of a field in one launch: the per-vector tests (validate.rs:59-78)
+// Validation of one TX x TY tile of a field in one launch: the per-vector tests (validate.rs:59-78)
 // on the tile and a halo of 3 cells, the normalized median test (:80-100) on the tile and a halo of
 // 2, the replacement by the median of usable neighbours at radius 1, then 2 (:102-128) on the tile,
 // and on the last pass the summary counts (:40-46). The flag snapshots between the stages stay in
-// shared memory; the halo cells are computed again by each tile that needs them (TY = 32: 1.27
-// times the median tests of separate launches; TY = 8: 1.69 times).
+// shared memory; the halo cells are computed again by each tile that needs them (32 x 32: 1.27 times
+// the median tests of separate launches; 32 x 8: 1.69 times).
 //
 // The stages are short and their launches were not: as three kernels with flag planes in memory and
 // two more for the summary, each pass of a small field spent 13 us in them and the last one 6 us
 // more (31 x 31 cells, B200); a 512 x 512 pair of one pass went from 48.6 to 39.1 us and a
 // batch of 64 pairs of 1280 x 800 from 4.17 to 3.76 ms with this and the export below.
-constexpr int kTileX = 32;
+//
+// The median and replacement loops walk only the cells that lie in the field, so that a tile of few
+// columns keeps its warps full: a warp that replaces one cell takes as long as one that replaces 32.
 constexpr int kValidateThreads = 256;
 
-template <int TY>
+template <int TX, int TY>
 __global__ void __launch_bounds__(kValidateThreads) validate_kernel(const __grid_constant__ ValidateBatch b) {
-    constexpr int LX = kTileX + 6, LY = TY + 6;  // values and first flags
-    constexpr int MX = kTileX + 4, MY = TY + 4;  // flags after the median test
+    constexpr int LX = TX + 6, LY = TY + 6;  // values and first flags
+    constexpr int MX = TX + 4, MY = TY + 4;  // flags after the median test
     __shared__ float su[LY][LX], sv[LY][LX];
     __shared__ uint8_t s1[LY][LX], s2[MY][MX];
     __shared__ unsigned int s_count[5];
@@ -276,8 +278,8 @@ __global__ void __launch_bounds__(kValidateThreads) validate_kernel(const __grid
     let_dependents_start();
     const int it = batch_item(b.tile_start, b.n, (int)blockIdx.x);
     const ValidateParams& p = b.item[it];
-    const int tile = (int)blockIdx.x - b.tile_start[it], tiles_x = (p.nx + kTileX - 1) / kTileX;
-    const int x0 = (tile % tiles_x) * kTileX, y0 = (tile / tiles_x) * TY;
+    const int tile = (int)blockIdx.x - b.tile_start[it], tiles_x = (p.nx + TX - 1) / TX;
+    const int x0 = (tile % tiles_x) * TX, y0 = (tile / tiles_x) * TY;
     if (threadIdx.x < 5) s_count[threadIdx.x] = 0;
     for (int i = threadIdx.x; i < LX * LY; i += kValidateThreads) {
         const int ly = i / LX, lx = i - ly * LX, x = x0 + lx - 3, y = y0 + ly - 3;
@@ -297,9 +299,13 @@ __global__ void __launch_bounds__(kValidateThreads) validate_kernel(const __grid
         sv[ly][lx] = v;
         s1[ly][lx] = f;
     }
+    for (int i = threadIdx.x; i < MX * MY; i += kValidateThreads) s2[i / MX][i % MX] = F_NO_SIGNAL;
     __syncthreads();
-    for (int i = threadIdx.x; i < MX * MY; i += kValidateThreads) {
-        const int my = i / MX, mx = i - my * MX, ly = my + 1, lx = mx + 1;
+    const int mx0 = max(2 - x0, 0), my0 = max(2 - y0, 0);  // first of s2's columns and rows in the field
+    const unsigned mw = min(p.nx - x0 + 2, MX) - mx0, mh = min(p.ny - y0 + 2, MY) - my0;
+    for (unsigned i = threadIdx.x; i < mw * mh; i += kValidateThreads) {
+        const unsigned row = mw == MX ? i / MX : i / mw;  // whole tiles divide by a constant
+        const int my = my0 + row, mx = mx0 + i - row * mw, ly = my + 1, lx = mx + 1;
         uint8_t f = s1[ly][lx];
         if ((f & F_INVALID) == 0) {
             // usable 3x3 neighbours (validate.rs:133-155), padded slots for the others
@@ -325,9 +331,11 @@ __global__ void __launch_bounds__(kValidateThreads) validate_kernel(const __grid
         s2[my][mx] = f;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kTileX * TY; i += kValidateThreads) {
-        const int ty = i / kTileX, tx = i % kTileX, x = x0 + tx, y = y0 + ty;
-        const bool in = x < p.nx && y < p.ny;
+    const unsigned w = min(p.nx - x0, TX), h = min(p.ny - y0, TY);
+    for (unsigned i0 = 0; i0 < w * h; i0 += kValidateThreads) {
+        const unsigned i = i0 + threadIdx.x;
+        const int ty = w == TX ? i / TX : i / w, tx = i - ty * w, x = x0 + tx, y = y0 + ty;
+        const bool in = i < w * h;
         uint8_t f = 0;
         if (in) {
             f = s2[ty + 2][tx + 2];
@@ -371,28 +379,52 @@ __global__ void __launch_bounds__(kValidateThreads) validate_kernel(const __grid
         atomicAdd(&p.counts[threadIdx.x], (unsigned long long)s_count[threadIdx.x]);
 }
 
-// Tile height: 32 rows when the batch then still has two tiles per SM, else 8 (a field of 31 x 31
-// cells is 4 tiles of 8 rows; 1000 x 1000 cells are 1024 tiles of 32).
-constexpr long long kTallTileCells = 148ll * 2 * kTileX * 32;
+struct ValidateTile {
+    int x, y;
+    void (*kernel)(ValidateBatch);
+};
+
+// The tile by the cells of the batch and its largest extents (us per call on fields of noise, B200, beside
+// the three separate launches that this kernel replaced):
+//   - few cells want many tiles, many cells little halo. 511 x 511: 32 x 8 35, 32 x 16 43, 32 x 32 44,
+//     separate 41; 660 x 660: 49, 47, 52, 50; 1021 x 1021: 100, 93, 100, 89; 1440 x 1440: 190, 167, 164, 162;
+//   - a field of few columns or rows fills only part of those tiles. 262,144 x 8 cells: 248, 205, 189, and
+//     158 in 16 x 64 (separate 158); 262,144 x 1: 146, 92, 66, and 25 in 4 x 128 (separate 25); 1 x 262,144:
+//     42 in 32 x 8 and 22 in 128 x 4 (separate 23); 16 x 131,072: 175 in 32 x 8, 149 in 64 x 16 (157). Below 32,768 cells no shape takes more than 22 us.
+ValidateTile validate_tile(const ValidateParams* items, int n) {
+    long long cells = 0;
+    int nx = 0, ny = 0;
+    for (int i = 0; i < n; ++i) {
+        cells += (long long)items[i].nx * items[i].ny;
+        nx = max(nx, items[i].nx);
+        ny = max(ny, items[i].ny);
+    }
+    if (cells >= 32768) {
+        if (nx <= 2) return {4, 128, validate_kernel<4, 128>};
+        if (ny <= 2) return {128, 4, validate_kernel<128, 4>};
+        if (nx <= (cells >= 400000 ? 16 : 4)) return {16, 64, validate_kernel<16, 64>};
+    }
+    if (cells < 400000) return {32, 8, validate_kernel<32, 8>};
+    if (ny <= 16) return {64, 16, validate_kernel<64, 16>};
+    if (cells < 1400000) return {32, 16, validate_kernel<32, 16>};
+    return {32, 32, validate_kernel<32, 32>};
+}
 
 cudaError_t launch_validate_items(const ValidateParams* items, int count, cudaStream_t s, int* launches) {
     for (int off = 0; off < count; off += kMaxBatch) {
         ValidateBatch b;
         b.n = min(count - off, kMaxBatch);
-        long long cells = 0;
-        for (int i = 0; i < b.n; ++i) cells += (long long)items[off + i].nx * items[off + i].ny;
-        const int ty = cells >= kTallTileCells ? 32 : 8;
+        const ValidateTile t = validate_tile(items + off, b.n);
         long long total = 0;
         for (int i = 0; i < b.n; ++i) {
             b.item[i] = items[off + i];
             b.tile_start[i] = (int)total;
-            total += (long long)((b.item[i].nx + kTileX - 1) / kTileX) * ((b.item[i].ny + ty - 1) / ty);
+            total += (long long)((b.item[i].nx + t.x - 1) / t.x) * ((b.item[i].ny + t.y - 1) / t.y);
         }
         b.tile_start[b.n] = (int)total;
         if (total <= 0) continue;
         if (total > 0x7fffffffll) return cudaErrorInvalidValue;
-        const cudaError_t e = launch_dependent(ty == 32 ? validate_kernel<32> : validate_kernel<8>, (unsigned)total,
-                                               kValidateThreads, 0, s, b);
+        const cudaError_t e = launch_dependent(t.kernel, (unsigned)total, kValidateThreads, 0, s, b);
         if (e != cudaSuccess) return e;
         if (launches) ++*launches;
     }
