@@ -40,21 +40,19 @@ struct BlurKernel {
 // inside it, sel[2] = clip code, sel[3] = blocks finished; all zeroed before level 0.
 //
 // Bound by launches and by the latency of the selection, not by its bytes: as separate kernels, each
-// selection walked its 256 bins in one thread (4 us). Codes come 16 bytes per load; level 0 counts
-// finer bins (code / 16) and adds them up at the end, as the codes of a camera fill few high bytes
-// (no difference within 1 us at 12 bits). Whole preparation with clip, per frame, B200: 1024 x 1024
-// u16 28.0 -> 16.4 us, u8 53.7 -> 12.8, 4096 x 4096 u16 65 -> 53.
+// selection walked its 256 bins in one thread (4 us). Codes come 16 bytes per load. Finer bins at level 0
+// (code / 16, added up at the end) gain nothing, not even where all codes share one high byte, and cost a
+// small frame 1 us (512 x 512 13.3 us against 14.3). Whole preparation with clip, per frame, B200: 1024 x
+// 1024 u16 28.0 -> 16.4 us, u8 53.7 -> 12.8, 4096 x 4096 u16 65 -> 52.
 constexpr int kHistThreads = 256;
 
 template <typename CodeT, int LEVEL>
 __global__ void __launch_bounds__(kHistThreads) hist_kernel(const CodeT* raw, long long n, unsigned int* hist,
                                                             unsigned int* sel, unsigned long long target) {
-    constexpr int kShift = 4;  // level 0 counts bins of code / 2^kShift
-    constexpr int kBins = LEVEL == 0 ? 65536 >> kShift : 256;
     constexpr int V = 16 / (int)sizeof(CodeT);
-    __shared__ unsigned int h[kBins];
+    __shared__ unsigned int h[kHistThreads];  // a bin per thread
     __shared__ bool last;
-    for (int i = threadIdx.x; i < kBins; i += kHistThreads) h[i] = 0;
+    h[threadIdx.x] = 0;
     __syncthreads();
     dependent_wait();
     let_dependents_start();
@@ -62,7 +60,7 @@ __global__ void __launch_bounds__(kHistThreads) hist_kernel(const CodeT* raw, lo
     const unsigned int coarse = LEVEL && !kOneByte ? sel[0] : 0u;
     auto count = [&](unsigned int c) {
         if (LEVEL == 0)
-            atomicAdd(&h[c >> kShift], 1u);
+            atomicAdd(&h[c >> 8], 1u);
         else if ((c >> 8) == coarse)
             atomicAdd(&h[c & 255u], 1u);
     };
@@ -84,15 +82,7 @@ __global__ void __launch_bounds__(kHistThreads) hist_kernel(const CodeT* raw, lo
     for (long long i = head + tid; i < n; i += stride) count(raw[i]);
     __syncthreads();
     unsigned int* const out = hist + 256 * LEVEL;
-    if constexpr (LEVEL == 0) {
-        constexpr int kFine = kBins / 256;
-        unsigned int v = 0;
-#pragma unroll
-        for (int k = 0; k < kFine; ++k) v += h[kFine * threadIdx.x + (k + threadIdx.x) % kFine];
-        if (v) atomicAdd(&out[threadIdx.x], v);
-    } else {
-        if (h[threadIdx.x]) atomicAdd(&out[threadIdx.x], h[threadIdx.x]);
-    }
+    if (h[threadIdx.x]) atomicAdd(&out[threadIdx.x], h[threadIdx.x]);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(&sel[3], 1u) == gridDim.x - 1;
