@@ -922,17 +922,17 @@ struct CorrVariant {
 
 #define PIV_V(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB, &launch_t<CorrCfg<N, T, PR, G, MB>>, &launch_t<CorrCfg<N, T, PR, G, MB>>}
 // the default variants have a kernel of their own for whole-pixel windows
-#define PIV_W(N, T, PR, G, MB, CG, CMB) \
-    {#N "/T" #T "/G" #G "/B" #MB, &launch_t<CorrCfg<N, T, PR, G, MB>>, &launch_t<CorrCfg<N, T, PR, CG, CMB, false, true>>}
-static const CorrVariant kV8[] = {PIV_W(8, 1, true, 16, 6, 16, 6), PIV_V(8, 1, true, 32, 3), PIV_V(8, 1, true, 32, 4)};
-static const CorrVariant kV12[] = {PIV_W(12, 1, true, 16, 4, 16, 4), PIV_V(12, 1, true, 16, 3), PIV_V(12, 1, true, 8, 6)};
-static const CorrVariant kV16[] = {PIV_W(16, 1, true, 16, 2, 16, 2), PIV_V(16, 1, true, 8, 4), PIV_V(16, 1, true, 8, 5)};
-static const CorrVariant kV24[] = {PIV_W(24, 2, true, 2, 6, 2, 6), PIV_V(24, 2, true, 4, 3), PIV_V(24, 2, true, 2, 4)};
-static const CorrVariant kV32[] = {PIV_W(32, 2, true, 4, 2, 4, 2), PIV_V(32, 2, true, 2, 4), PIV_V(32, 2, true, 1, 8)};
-static const CorrVariant kV48[] = {PIV_W(48, 4, true, 1, 3, 1, 3), PIV_V(48, 4, true, 1, 2)};
-static const CorrVariant kV64[] = {PIV_W(64, 4, true, 1, 2, 1, 2), PIV_V(64, 4, true, 1, 1)};
-static const CorrVariant kV96[] = {PIV_W(96, 4, true, 1, 1, 1, 1)};
-static const CorrVariant kV128[] = {PIV_W(128, 4, false, 1, 1, 1, 1)};
+#define PIV_W(N, T, PR, G, MB) \
+    {#N "/T" #T "/G" #G "/B" #MB, &launch_t<CorrCfg<N, T, PR, G, MB>>, &launch_t<CorrCfg<N, T, PR, G, MB, false, true>>}
+static const CorrVariant kV8[] = {PIV_W(8, 1, true, 16, 6), PIV_V(8, 1, true, 32, 3), PIV_V(8, 1, true, 32, 4)};
+static const CorrVariant kV12[] = {PIV_W(12, 1, true, 16, 4), PIV_V(12, 1, true, 16, 3), PIV_V(12, 1, true, 8, 6)};
+static const CorrVariant kV16[] = {PIV_W(16, 1, true, 16, 2), PIV_V(16, 1, true, 8, 4), PIV_V(16, 1, true, 8, 5)};
+static const CorrVariant kV24[] = {PIV_W(24, 2, true, 2, 6), PIV_V(24, 2, true, 4, 3), PIV_V(24, 2, true, 2, 4)};
+static const CorrVariant kV32[] = {PIV_W(32, 2, true, 4, 2), PIV_V(32, 2, true, 2, 4), PIV_V(32, 2, true, 1, 8)};
+static const CorrVariant kV48[] = {PIV_W(48, 4, true, 1, 3), PIV_V(48, 4, true, 1, 2)};
+static const CorrVariant kV64[] = {PIV_W(64, 4, true, 1, 2), PIV_V(64, 4, true, 1, 1)};
+static const CorrVariant kV96[] = {PIV_W(96, 4, true, 1, 1)};
+static const CorrVariant kV128[] = {PIV_W(128, 4, false, 1, 1)};
 // Deformed-window variants: the same FFT decomposition per size, the deformed sampler.
 #define PIV_D(N, T, PR, G, MB) {#N "/T" #T "/G" #G "/B" #MB "/deform", &launch_t<CorrCfg<N, T, PR, G, MB, true>>, nullptr}
 static const CorrVariant kD8[] = {PIV_D(8, 1, true, 32, 3)};
