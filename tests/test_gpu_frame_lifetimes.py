@@ -136,3 +136,42 @@ def test_blocks_of_dropped_frames_wait_for_queued_work(stream):
             assert np.array_equal(fl.cpu().numpy(), want.flags)
             [t.zero_() for t in (*out, fl)]
             torch.cuda.synchronize()
+
+
+def test_a_callers_captured_analysis_replays_while_frames_come_and_go():
+    """Work captured by the caller may run at any later time: what it uses stays its own."""
+    import torch
+
+    import piv_b200 as P
+    h, w = 192, 256
+    an = P.PivAnalyzer(_config())
+    s = torch.cuda.Stream()
+    an.set_stream(s.cuda_stream)
+    raw = [torch.from_numpy(i).cuda() for i in _images(5, h, w)]
+    fa, fb = an.frame(h, w), an.frame(h, w)
+    n = an.output_grid(h, w)
+    out = [torch.zeros(n.ny, n.nx, device="cuda") for _ in range(3)]
+    fl = torch.zeros(n.ny, n.nx, device="cuda", dtype=torch.uint8)
+
+    def work():
+        fa.prepare_device(raw[0].data_ptr(), P.api._lib.PIV_DTYPE_F32, P.PreprocessConfig())
+        fb.prepare_device(raw[1].data_ptr(), P.api._lib.PIV_DTYPE_F32, P.PreprocessConfig())
+        an.analyze_device(fa, fb, *[t.data_ptr() for t in out], fl.data_ptr())
+
+    torch.cuda.synchronize()
+    work()  # allocates
+    an.sync()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        work()
+    for seed in (5, 6, 7):
+        a, b = _images(seed, h, w)
+        ref = P.PivAnalyzer(_config())
+        want = ref.analyze(ref.prepare(a), ref.prepare(b)).field  # its frames are dropped at once
+        with torch.cuda.stream(s):
+            raw[0].copy_(torch.from_numpy(a))
+            raw[1].copy_(torch.from_numpy(b))
+            g.replay()
+        s.synchronize()
+        assert same_floats(out[0].cpu().numpy(), want.dx) and same_floats(out[1].cpu().numpy(), want.dy)
+        assert same_floats(out[2].cpu().numpy(), want.peak_ratio) and np.array_equal(fl.cpu().numpy(), want.flags)
