@@ -215,13 +215,12 @@ bool wait_call(CallLog& log, uint64_t c) {
     std::unique_lock<std::mutex> lk(log.mu);
     if (log.completed(c)) return true;
     if (log.lost(c)) return false;
-    uint64_t n = 0;
+    uint64_t n = c;  // a later call may have been counted and not queued yet: it is not waited for
     cudaError_t e = cudaErrorUnknown;
     if (log.on_own && log.own) {
         cudaEvent_t ev = nullptr;
         if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess) {
             e = cudaEventRecord(ev, log.own);
-            n = log.calls;
             lk.unlock();
             if (e == cudaSuccess) e = cudaEventSynchronize(ev);
             cudaEventDestroy(ev);
@@ -444,8 +443,9 @@ uint64_t begin_call(PivAnalyzer* an, std::initializer_list<const PivFrame*> fram
         call = ++an->log->calls;
         if (!an->log->on_own) {  // a caller's capture: its graph may run at any later time
             cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(an->cur, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-                an->log->lose_pending();
+            const cudaError_t e = cudaStreamIsCapturing(an->cur, &cap);
+            if (e != cudaSuccess) cudaGetLastError();
+            if (e != cudaSuccess || cap != cudaStreamCaptureStatusNone) an->log->lose_pending();
         }
     }
     for (const PivFrame* f : frames)
