@@ -889,7 +889,8 @@ int prepare_common(PivAnalyzer* an, PivFrame* f, const void* raw_dev, int32_t dt
 }
 
 // prepare_common for frames of one size and type: plain conversions (no clip, blur, normalisation or
-// mask tables) of all frames go in one launch.
+// mask tables) of all frames go in one launch. f32 frames have no plain form: they may hold negative
+// samples, so they need the mask tables (only a background subtracted from them would spare those).
 int prepare_frames(PivAnalyzer* an, PivFrame* const* frames, const void* const* raw_dev, int count, int32_t dtype,
                    const PivPreprocessC* pre, const float* bg_dev) {
     const bool plain = dtype != PIV_DTYPE_F32 && pre && !(pre->clip_percentile > 0.0) && !(pre->smooth_sigma > 0.0f) &&
